@@ -2,8 +2,8 @@
 // of one network (replaces GGASolver.__init__'s index build,
 // dgga/solver.py:239-369, and symbolic.build_symbolic, dgga/symbolic.py:475).
 //
-//  * ordering: minimum degree on the elimination graph (ties broken by the
-//    smallest junction row), or a caller-supplied permutation;
+//  * ordering: depth-aware minimum degree on the elimination graph (few
+//    dependent levels), or a caller-supplied permutation;
 //  * elimination tree and the structure of L by merging children's column
 //    structures; columns scheduled by elimination-tree level (leaves first);
 //  * left-looking LDL^T task lists: one task per entry of L, each a list of
@@ -31,15 +31,27 @@ int fail(int code, const std::string& msg) {
   return code;
 }
 
-// Minimum-degree ordering on the explicit elimination graph.
+// Depth-aware minimum-degree ordering on the explicit elimination graph.  A
+// junction's elimination level is one more than the largest level among the
+// neighbours eliminated before it; the next junction is the one with the
+// smallest 2 degree + level (ties by the smallest row).  The kernels run one
+// dependent step per level, so a chain of degree-2 junctions eliminated one
+// after the other, which plain minimum degree does when ties go by row, costs
+// a step per junction; the level term spreads the elimination over the graph
+// instead, for a few per cent more entries.  Levels below the dense top block
+// / entries of L, plain minimum degree -> this: 100 junctions 3 / 289 -> 2 /
+// 294; 542 with 79 TCVs 20 / 1229 -> 5 / 1336; 782 17 / 2327 -> 7 / 2397;
+// 3000 36 / 9922 -> 18 / 10155; 20 000 66 / 63 359 -> 40 / 64 982.  Weights
+// of 1/4 and 1 on the level leave more levels or more entries.
 std::vector<int> min_degree(int n, std::vector<std::vector<int>> adj) {
-  std::vector<int> deg(n), order;
+  std::vector<int> deg(n), lev(n, 0), order;
   order.reserve(n);
   std::vector<char> alive(n, 1);
   std::set<std::pair<int, int>> pq;
+  auto key = [&](int i) { return std::make_pair(2 * deg[i] + lev[i], i); };
   for (int i = 0; i < n; ++i) {
     deg[i] = (int)adj[i].size();
-    pq.insert({deg[i], i});
+    pq.insert(key(i));
   }
   std::vector<int> merged;
   while (!pq.empty()) {
@@ -51,7 +63,7 @@ std::vector<int> min_degree(int n, std::vector<std::vector<int>> adj) {
     for (int u : adj[v])
       if (alive[u]) nb.push_back(u);
     for (int u : nb) {
-      pq.erase({deg[u], u});
+      pq.erase(key(u));
       merged.clear();
       std::set_union(adj[u].begin(), adj[u].end(), nb.begin(), nb.end(),
                      std::back_inserter(merged));
@@ -61,7 +73,8 @@ std::vector<int> min_degree(int n, std::vector<std::vector<int>> adj) {
         if (w != u && alive[w]) nu.push_back(w);
       adj[u].swap(nu);
       deg[u] = (int)adj[u].size();
-      pq.insert({deg[u], u});
+      lev[u] = std::max(lev[u], lev[v] + 1);
+      pq.insert(key(u));
     }
     adj[v].clear();
   }
