@@ -58,8 +58,8 @@ struct Sh {
   float* Wf;                      // the factor when it is kept in FP32 (W is then null)
   double *em_e, *em_ke, *em_emh;  // per emitter slot: flow, coefficient, 1/hgrad
   int16_t* eslot;                 // [Nj] emitter slot of a junction or -1
-  double* tb;                     // [2][49] pivot columns (+ 1/pivot) of the top-block inversion
-  double* Mg;                     // [nT][nT] top-block inverse (global workspace)
+  double* tb;                     // scratch of the top-block inversion (V2's storage)
+  double* Mg;                     // [nT][top_ld(nT)] top-block inverse (shared memory when n.msm, else global)
   int *wcnt, *flag, *err;
   int8_t* S;
 };
@@ -625,148 +625,243 @@ __device__ __forceinline__ double pow2_scale(double x) {
   return __longlong_as_double((1023 - h) << 52);
 }
 
-// One sweep of the top-block inversion (see top_inverse) for pivot k, which
-// lies in register block KB; NJ is the register block of column k + 1 and PAR
-// the parity of k (the buffer that holds column k).  All three are static,
-// so that no register is selected at run time.
-template <int NT, int KB, int NJ, int PAR>
-__device__ __forceinline__ void top_sweep(int k, int nT, int r, int c, double (&a)[3][3],
-                                          double* tb, int& bad) {
-  constexpr int ST = WDS_TOP_MAX + 1;
-  const double* cb = tb + PAR * ST;
-  double* nb = tb + (1 - PAR) * ST;
-  const double ip = cb[WDS_TOP_MAX];
-  const double c0 = cb[c], c1 = cb[c + 16], c2 = cb[c + 32];
-#pragma unroll
-  for (int ia = 0; ia < 3; ++ia) {
-    const double t = cb[r + 16 * ia] * ip;
-    a[ia][0] = fma(-t, c0, a[ia][0]);
-    a[ia][1] = fma(-t, c1, a[ia][1]);
-    a[ia][2] = fma(-t, c2, a[ia][2]);
-  }
-  const int km = k & 15;
-  if (r == km && c == km) a[KB][KB] = -ip;  // the pivot: a_kk = -1/p
-  // publish column kn = k + 1 (all rows: the full matrix is kept), then
-  // p - 1 at its pivot and 1/p
-  const int kn = k + 1, kq = kn & 15;
-  if (kn < nT && c == kq) {
-    nb[r] = a[0][NJ];
-    nb[r + 16] = a[1][NJ];
-    nb[r + 32] = a[2][NJ];
-    if (r == kq) {
-      const double x = a[NJ][NJ];
-      if (!(x > 0.0) || !isfinite(x)) bad = 1;
-      nb[WDS_TOP_MAX] = __drcp_rn(x);
-      nb[kn] = x - 1.0;
-    }
-  }
-  gsync<NT>();
+// One double-precision tensor-core product: c += a b^T on an 8 x 8 tile, four
+// columns deep (lane l holds a[l / 4][l % 4], b[l / 4][l % 4] and
+// c[l / 4][2 (l % 4) + {0, 1}]).
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
 }
 
-// The sweeps k in [16 KB, min(16 KB + 16, nT)): in pairs (static parity);
-// column k + 1 lies in block KB except after the block's last pivot.
-template <int NT, int KB>
-__device__ __forceinline__ void top_block(int nT, int r, int c, double (&a)[3][3], double* tb,
-                                          int& bad) {
-  const int k0 = 16 * KB;
-  if (k0 >= nT) return;
-  const int kend = min(k0 + 16, nT), kmid = min(k0 + 15, kend);
-  int k = k0;
-#pragma unroll 1
-  for (; k + 1 < kmid; k += 2) {
-    top_sweep<NT, KB, KB, 0>(k, nT, r, c, a, tb, bad);
-    top_sweep<NT, KB, KB, 1>(k + 1, nT, r, c, a, tb, bad);
+constexpr int kTopTiles = WDS_TOP_MAX / 8;   // 8 x 8 tiles along one side
+// One panel buffer of the inversion: the block's four columns [WDS_TOP_MAX][4],
+// then the inverse of its 4 x 4 pivot block
+constexpr int kTopPanel = 4 * WDS_TOP_MAX + 16;
+// Doubles of group scratch: three panel buffers and the row scales
+constexpr int kTopScratch = 3 * kTopPanel + WDS_TOP_MAX;
+
+// The inversion's two barriers (ids beside the groups' own): the `warps` warps
+// that hold tile rows hand a block's columns to the pivot warp (A) and take
+// its inverse back (B).  The producers of either only arrive.
+template <int NT>
+__device__ __forceinline__ void top_arrive(int id, int warps) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id + (int)(threadIdx.x / NT)), "r"(32 * warps + 32)
+               : "memory");
+}
+template <int NT>
+__device__ __forceinline__ void top_wait(int id, int warps) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id + (int)(threadIdx.x / NT)), "r"(32 * warps + 32)
+               : "memory");
+}
+constexpr int kTopA = 5, kTopB = 9;
+
+// 1 / x for a positive normal x to about one unit in the last place: the
+// hardware's 23-bit approximation and two Newton steps (48 cycles of latency
+// against 77 of the correctly rounded __drcp_rn, measured on dependent
+// chains).
+__device__ __forceinline__ double recip(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+
+// Inverse of the 4 x 4 pivot block at q (row-major), every lane the same (so
+// that nothing is broadcast); lane 0 writes it to pin.  The pivots come in pairs with one reciprocal each:
+// d1 = a, d1 d2 = a d - b^2 (with the product's rounding error compensated),
+// 1 / d1 = det r and 1 / d2 = a^2 r with r = 1 / (a det).
+__device__ __forceinline__ void top_pivot(const double* q, double* pin, int lane, int& bad) {
+  const double a11 = q[0], a21 = q[4], a22 = q[5];
+  const double w1 = a21 * a21;
+  const double det1 = fma(a11, a22, -w1) - fma(a21, a21, -w1);
+  const double r1 = recip(a11 * det1);
+  const double i1 = det1 * r1, i2 = a11 * a11 * r1;
+  const double l21 = a21 * i1;
+  const double a31 = q[8], l31 = a31 * i1;
+  const double b32 = fma(-l31, a21, q[9]), l32 = b32 * i2;
+  const double c33 = fma(-l32, b32, fma(-l31, a31, q[10]));
+  const double a41 = q[12], l41 = a41 * i1;
+  const double b42 = fma(-l41, a21, q[13]), l42 = b42 * i2;
+  const double c43 = fma(-l42, b32, fma(-l41, a31, q[14]));
+  const double c44 = fma(-l42, b42, fma(-l41, a41, q[15]));
+  const double w2 = c43 * c43;
+  const double det2 = fma(c33, c44, -w2) - fma(c43, c43, -w2);
+  const double r2 = recip(c33 * det2);
+  const double i3 = det2 * r2, i4 = c33 * c33 * r2;
+  const double l43 = c43 * i3;
+  if (!(a11 > 0.0) || !(det1 > 0.0) || !(c33 > 0.0) || !(det2 > 0.0) || !isfinite(det1) ||
+      !isfinite(det2))
+    bad = 1;
+  // rows of L^-1 (unit lower), then L^-T D^-1 L^-1 from its last row up
+  const double m31 = fma(l32, l21, -l31), m42 = fma(l43, l32, -l42);
+  const double m41 = -fma(l43, m31, fma(-l42, l21, l41));
+  const double p43 = -l43 * i4, p42 = m42 * i4, p41 = m41 * i4;
+  const double e32 = -l32 * i3, e31 = m31 * i3, e21 = -l21 * i2;
+  const double p33 = fma(-l43, p43, i3), p32 = fma(-l43, p42, e32), p31 = fma(-l43, p41, e31);
+  const double p22 = fma(m42, p42, fma(-l32, e32, i2));
+  const double p21 = fma(m42, p41, fma(-l32, e31, e21));
+  const double p11 = fma(m41, p41, fma(m31, e31, fma(-l21, e21, i1)));
+  if (lane == 0) {
+    double2* o = reinterpret_cast<double2*>(pin);
+    o[0] = make_double2(p11, p21);
+    o[1] = make_double2(p31, p41);
+    o[2] = make_double2(p21, p22);
+    o[3] = make_double2(p32, p42);
+    o[4] = make_double2(p31, p32);
+    o[5] = make_double2(p33, p43);
+    o[6] = make_double2(p41, p42);
+    o[7] = make_double2(p43, i4);
   }
-  if (k < kmid) top_sweep<NT, KB, KB, 0>(k, nT, r, c, a, tb, bad);
-  if (k0 + 15 < kend) top_sweep<NT, KB, (KB < 2 ? KB + 1 : KB), 1>(k0 + 15, nT, r, c, a, tb, bad);
+}
+
+// Publishes the four columns of block K from the tiles (their rows in every
+// warp).
+template <int K>
+__device__ __forceinline__ void top_publish(int w, int lane, const double (&c)[kTopTiles][2],
+                                            double* tb) {
+  if (((lane & 3) >> 1) == (K & 1))
+    *reinterpret_cast<double2*>(tb + (K % 3) * kTopPanel + (8 * w + (lane >> 2)) * 4 +
+                                2 * (lane & 1)) = make_double2(c[K >> 1][0], c[K >> 1][1]);
+}
+
+// Block K of the inversion on a tile-row warp: every tile takes the block's
+// rank-4 update, the tile that holds the next block's columns first, so that
+// those go out (and the pivot warp inverts their pivot block) while the other
+// tiles are still updated.
+template <int NT, int K>
+__device__ __forceinline__ void top_steps(int nT, int tiles, int w, int lane,
+                                          double (&c)[kTopTiles][2], double* tb) {
+  if constexpr (4 * K < WDS_TOP_MAX) {
+    if (4 * K >= nT) return;
+    constexpr int tK = K >> 1, tN = (K + 1) >> 1 < kTopTiles ? (K + 1) >> 1 : tK;
+    const double* buf = tb + (K % 3) * kTopPanel;
+    const double* pin = buf + 4 * WDS_TOP_MAX;
+    const int i = lane >> 2, m = lane & 3;
+    // this lane's row of its tile row (prow, when w == tK) and of tile tK's
+    // columns lies in the pivot block, at (i % 4, m)
+    const bool prow = (i >> 2) == (K & 1);
+    const double one = prow && (i & 3) == m ? 1.0 : 0.0;
+    top_wait<NT>(kTopB, tiles);
+    const double2* u = reinterpret_cast<const double2*>(buf + (8 * w + i) * 4);
+    const double2* pv = reinterpret_cast<const double2*>(pin + 4 * m);
+    const double2 u0 = u[0], u1 = u[1], p0 = pv[0], p1 = pv[1];
+    const double pim = pin[4 * (i & 3) + m];
+    const double2 pk = *reinterpret_cast<const double2*>(pin + 4 * (i & 3) + 2 * (m & 1));
+    double bN = buf[(8 * tN + i) * 4 + m];
+    if (tN == tK) bN -= one;  // P - I
+    // -T, T = U P^-1; its pivot rows are I - P^-1
+    double a = -fma(u1.y, p1.y, fma(u1.x, p1.x, fma(u0.y, p0.y, u0.x * p0.x)));
+    a = w == tK && prow ? pim - one : a;
+    const bool own = w == tK && prow && (m >> 1) == (K & 1);  // holds -P^-1 afterwards
+    auto tile = [&](int t, double b) {
+      dmma(c[t], a, b);
+      if (t == tK) {
+        c[t][0] = own ? -pk.x : c[t][0];
+        c[t][1] = own ? -pk.y : c[t][1];
+      }
+    };
+    tile(tN, bN);
+    if constexpr (4 * (K + 1) < WDS_TOP_MAX) {
+      if (4 * (K + 1) < nT) {
+        top_publish<K + 1>(w, lane, c, tb);
+        top_arrive<NT>(kTopA, tiles);
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < kTopTiles; ++t)
+      if (t != tN && t < tiles) tile(t, buf[(8 * t + i) * 4 + m] - (t == tK ? one : 0.0));
+    top_steps<NT, K + 1>(nT, tiles, w, lane, c, tb);
+  }
 }
 
 // Inverse of the top block's Schur complement S (nT x nT, nT <= WDS_TOP_MAX)
-// by symmetric sweeps (Gauss-Jordan elimination without pivoting, in column
-// order; every pivot is then a pivot of the LDL^T of S, so its sign is the
-// positive-definiteness check).  S is first scaled to S' = D S D with D the
-// power-of-two diagonal that brings diag(S') into [0.5, 2) (exact), so the
-// pivots p of S' are at most about 2, and S^{-1} = D S'^{-1} D.
-// Sweeping k maps a_kk -> -1/p, a_ik -> a_ik/p, a_kj -> a_kj/p and
-// a_ij -> a_ij - (a_ik/p) a_kj; after all nT sweeps the matrix is -S'^{-1}.
-// With the pivot's entry of the published column set to p - 1, the one
-// rank-1 update a_ij -> a_ij - (c_i/p) c_j (c = column k) gives row and
-// column k as well: c_i - (c_i/p)(p - 1) = c_i/p, without cancellation since
-// |p - 1| <= 1 after the scaling; only a_kk is then overwritten (-1/p).
-// Thread (r, c) of a 16 x 16 grid holds the entries (r + 16 a, c + 16 b),
-// a, b < 3, of the full matrix in registers for all sweeps, so that a sweep
-// is 6 shared loads, 3 multiplies and 9 FMAs per thread; the sweep's code is
-// instantiated per register block and buffer parity (top_block), so the
-// sweep is short: about 430 cycles alone against 530 with the block chosen
-// at run time.  Column k+1 after sweep k goes through shared memory: two
-// alternating buffers of 49 (the column, then 1/p of its pivot, which the
-// pivot's owner computes and checks) and one group barrier per sweep.  S is
-// read from the factor slots listed in dslot, S^{-1} is written to Mg
-// (row-major, each entry by its owner).  Returns 1 when this thread owned a
-// pivot that was not positive and finite.  Runs as a separate function so
-// that its block of registers does not add to the caller's.
+// by symmetric block sweeps (Gauss-Jordan elimination without pivoting, four
+// columns at a time in column order; the pivots of the 4 x 4 blocks are those
+// of the LDL^T of S, so their signs are the positive-definiteness check).  S
+// is first scaled to S' = D S D with D the power-of-two diagonal that brings
+// diag(S') into [0.5, 2) (exact), and S^{-1} = D S'^{-1} D.
+// Sweeping block k with pivot block P and columns U maps S_kk -> -P^-1,
+// S_ik -> U_i P^-1 and S_ij -> S_ij - U_i P^-1 U_j^T; after all blocks the
+// matrix is -S'^{-1}.  With P - I in the pivot rows of U the one rank-4 update
+// gives the block's rows and columns as well: U - (U P^-1)(P - I) = U P^-1,
+// without cancellation since the entries of P - I are at most about 2 after
+// the scaling; only S_kk is then overwritten.
+// Warp w holds tile row w (8 rows of the full matrix) in registers for all
+// blocks, six 8 x 8 tiles, and each tile's update is one m8n8k4 FP64
+// tensor-core product: a block costs a warp six of them and 4 FMAs per lane,
+// where four single-column sweeps on 3 x 3 entries per thread cost 48
+// multiplies and FMAs per lane and four barriers of the whole group.  A
+// seventh warp inverts the pivot blocks.  What bounds it is the chain of a
+// block: publish the columns, invert the 4 x 4 block (two reciprocals), read
+// it back, update the next block's tile.  S is read from the factor slots
+// listed in dslot, S^{-1} is written to Mg (row-major, rows of top_ld(nT)
+// entries); tb: kTopScratch doubles of the group (a panel buffer is written
+// again only when every warp is past its tiles two blocks before).  Returns 1
+// when this thread saw a pivot that was not positive and finite.  Runs as a
+// separate function so that its tiles do not add to the caller's registers.
 template <int NT, class Slot, class FT>
 __device__ __noinline__ int top_inverse(const FT* W, const Slot* dslot, double* tb,
                                         double* Mg, int nT) {
-  static_assert(NT == 256 && WDS_TOP_MAX == 48, "16 x 16 threads x 3 x 3 entries");
-  constexpr int ST = WDS_TOP_MAX + 1;
-  const int tid = gtid<NT>(), r = tid >> 4, c = tid & 15;
-  double a[3][3];
-  int bad = 0;
+  static_assert(NT >= 4 * WDS_TOP_MAX + 32 && WDS_TOP_MAX % 8 == 0,
+                "a warp per tile row and one for the pivots");
+  const int w = gtid<NT>() >> 5, lane = threadIdx.x & 31, i = lane >> 2, m = lane & 3;
+  const int tiles = (nT + 7) >> 3, r = 8 * w + i;
+  // the pivot warp: 6 or 7, so that neighbouring groups' lie on different
+  // SM sub-partitions
+  const int wp = kTopTiles + ((int)(threadIdx.x / NT) & 1);
+  if (w == wp) {
+    int bad = 0;
+    for (int k = 0, o = 0; 4 * k < nT; ++k, o = o == 2 * kTopPanel ? 0 : o + kTopPanel) {
+      top_wait<NT>(kTopA, tiles);
+      top_pivot(tb + o + 16 * k, tb + o + 4 * WDS_TOP_MAX, lane, bad);
+      top_arrive<NT>(kTopB, tiles);
+    }
+    return bad;
+  }
+  if (w >= tiles) return 0;
+  double c[kTopTiles][2];
 #pragma unroll
-  for (int ia = 0; ia < 3; ++ia)
+  for (int t = 0; t < kTopTiles; ++t)
 #pragma unroll
-    for (int jb = 0; jb < 3; ++jb) {
-      const int i = r + 16 * ia, j = c + 16 * jb;
-      double x = 0.0;
-      if (i < nT && j < nT) {
-        const int hi = i > j ? i : j, lo = i > j ? j : i;
+    for (int e = 0; e < 2; ++e) {
+      const int j = 8 * t + 2 * m + e;
+      double x = r == j ? 1.0 : 0.0;  // rows beyond nT: identity
+      if (r < nT && j < nT) {
+        const int hi = r > j ? r : j, lo = r > j ? j : r;
         const Slot sl = dslot[hi * (hi + 1) / 2 + lo];
-        if (sl != (Slot)~Slot(0)) x = (double)W[sl];
+        x = sl != (Slot)~Slot(0) ? (double)W[sl] : 0.0;
       }
-      a[ia][jb] = x;
+      c[t][e] = x;
     }
-  // the scale of row i goes through tb[ST + i] (the diagonal's owner writes it)
-  if (r == c) {
+  double* sc = tb + 3 * kTopPanel;
 #pragma unroll
-    for (int ia = 0; ia < 3; ++ia)
-      if (r + 16 * ia < nT) tb[ST + r + 16 * ia] = pow2_scale(a[ia][ia]);
-  }
-  gsync<NT>();
-  double dr[3], dc[3];
+  for (int t = 0; t < kTopTiles; ++t)
+    if (t == w && m == (i >> 1)) sc[r] = pow2_scale((i & 1) ? c[t][1] : c[t][0]);
+  asm volatile("bar.sync %0, %1;" ::"r"(kTopB + (int)(threadIdx.x / NT)), "r"(32 * tiles)
+               : "memory");
+  const double dr = sc[r];
 #pragma unroll
-  for (int ia = 0; ia < 3; ++ia) {
-    dr[ia] = r + 16 * ia < nT ? tb[ST + r + 16 * ia] : 1.0;
-    dc[ia] = c + 16 * ia < nT ? tb[ST + c + 16 * ia] : 1.0;
-  }
-#pragma unroll
-  for (int ia = 0; ia < 3; ++ia)
-#pragma unroll
-    for (int jb = 0; jb < 3; ++jb) a[ia][jb] *= dr[ia] * dc[jb];
-  gsync<NT>();
-  // column 0 (rows beyond nT are zero), then p - 1 at the pivot and 1/p
-  if (c == 0) {
-#pragma unroll
-    for (int ia = 0; ia < 3; ++ia) tb[r + 16 * ia] = a[ia][0];
-    if (r == 0) {
-      const double p = a[0][0];
-      if (!(p > 0.0) || !isfinite(p)) bad = 1;
-      tb[WDS_TOP_MAX] = __drcp_rn(p);
-      tb[0] = p - 1.0;
+  for (int t = 0; t < kTopTiles; ++t)
+    if (t < tiles) {
+      const double2 d = *reinterpret_cast<const double2*>(sc + 8 * t + 2 * m);
+      c[t][0] *= dr * d.x;
+      c[t][1] *= dr * d.y;
     }
-  }
-  gsync<NT>();
-  top_block<NT, 0>(nT, r, c, a, tb, bad);
-  top_block<NT, 1>(nT, r, c, a, tb, bad);
-  top_block<NT, 2>(nT, r, c, a, tb, bad);
+  top_publish<0>(w, lane, c, tb);
+  top_arrive<NT>(kTopA, tiles);
+  top_steps<NT, 0>(nT, tiles, w, lane, c, tb);
+  const int ld = top_ld(nT);
 #pragma unroll
-  for (int ia = 0; ia < 3; ++ia)
-#pragma unroll
-    for (int jb = 0; jb < 3; ++jb) {
-      const int i = r + 16 * ia, j = c + 16 * jb;
-      if (i < nT && j < nT) Mg[i * nT + j] = -a[ia][jb] * (dr[ia] * dc[jb]);
+  for (int t = 0; t < kTopTiles; ++t)
+    if (t < tiles) {
+      const double2 d = *reinterpret_cast<const double2*>(sc + 8 * t + 2 * m);
+      const int j = 8 * t + 2 * m;
+      if (r < nT && j < nT)
+        *reinterpret_cast<double2*>(Mg + r * ld + j) =
+            make_double2(-c[t][0] * (dr * d.x), -c[t][1] * (dr * d.y));
     }
-  return bad;
+  return 0;
 }
 
 template <int NT>
@@ -774,7 +869,7 @@ __device__ __noinline__ void top_apply(const double* Mg, double* vT, int nT) {
   const int tid = gtid<NT>(), i = tid >> 2, li = tid & 3;
   double acc0 = 0.0, acc1 = 0.0;
   if (i < nT) {
-    const double* row = Mg + i * nT;
+    const double* row = Mg + i * top_ld(nT);
 #pragma unroll
     for (int q = 0; q < WDS_TOP_MAX / 4; q += 2) {
       const int j0 = li + 4 * q, j1 = j0 + 4;
@@ -1299,6 +1394,11 @@ __device__ void primal_solve(const DevNet& n, const TB& T, const Sh& s, double* 
 
 __device__ __forceinline__ size_t al16(size_t x) { return (x + 15) / 16 * 16; }
 
+// doubles of V2: a node vector, or the top-block inversion's scratch
+__host__ __device__ inline int v2_len(const DevNet& n) {
+  return n.nT > 0 && n.Nj < kTopScratch ? kTopScratch : n.Nj;
+}
+
 __device__ Sh carve(const DevNet& n, unsigned char* base) {
   Sh s;
   size_t o = 0;
@@ -1315,7 +1415,10 @@ __device__ Sh carve(const DevNet& n, unsigned char* base) {
   }
   s.V0 = (double*)take(8ull * n.Nj);
   s.V1 = (double*)take(8ull * n.Nj);
-  s.V2 = (double*)take(8ull * n.Nj);
+  // the solves' temporary; idle while the matrix is factored, so the top
+  // block's inversion works there
+  s.V2 = (double*)take(8ull * v2_len(n));
+  s.tb = s.V2;
   s.em_e = (double*)take(8ull * n.emcap);
   s.em_ke = (double*)take(8ull * n.emcap);
   s.em_emh = (double*)take(8ull * n.emcap);
@@ -1324,8 +1427,9 @@ __device__ Sh carve(const DevNet& n, unsigned char* base) {
   s.red = (double*)take(8ull * 4 * 32);
   s.small = (double*)take(8ull * (4 * n.npcv * n.npcv + 5 * n.npcv + 8));
   s.eslot = (int16_t*)take(2ull * n.Nj);
-  s.tb = (double*)take(8ull * 2 * (WDS_TOP_MAX + 1));
-  s.Mg = nullptr;  // set by the kernel
+  // the top block's inverse, where it fits (else the kernel points it to the
+  // scenario's slice of the global workspace)
+  s.Mg = n.msm ? (double*)take(8ull * n.nT * top_ld(n.nT)) : nullptr;
   s.wcnt = (int*)take(4ull * 32);
   s.flag = (int*)take(16);      // [0] factor verdict, [1] error, [2] emitter count
   s.err = s.flag + 1;
@@ -1338,14 +1442,14 @@ size_t smem_bytes(const DevNet& n) {
   size_t o = 0;
   o += a16(8ull * n.L);
   o += a16((n.fp32 ? 4ull : 8ull) * n.nnzL);
-  o += 3 * a16(8ull * n.Nj);
+  o += 2 * a16(8ull * n.Nj) + a16(8ull * v2_len(n));
   o += 3 * a16(8ull * n.emcap);
   o += a16(8ull * (n.Nf > 0 ? n.Nf : 1));
   o += a16(8ull * (n.nxf > 0 ? n.nxf : 1));
   o += a16(8ull * 4 * 32);
   o += a16(8ull * (4 * n.npcv * n.npcv + 5 * n.npcv + 8));
   o += a16(2ull * n.Nj);
-  o += a16(8ull * 2 * (WDS_TOP_MAX + 1));
+  if (n.msm) o += a16(8ull * n.nT * top_ld(n.nT));
   o += a16(4ull * 32);
   o += a16(16);
   o += a16(n.L);
@@ -1443,7 +1547,7 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
                                             const TB& T, Sh s, int b) {
   s.q = w.lk + (size_t)b * 2 * n.L;
   s.Y = s.q + n.L;
-  s.Mg = w.M + (size_t)b * n.nT * n.nT;
+  if (!n.msm) s.Mg = w.M + (size_t)b * n.nT * top_ld(n.nT);
   const double* rrow = a.r + (long long)b * a.r_stride;
   const double* kerow = a.ke + (long long)b * a.ke_stride;
   const double* drow = a.d + (long long)b * n.N;
@@ -1806,6 +1910,10 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
     if (info == 0) {  // store the terminal state for the adjoint
       FT* Wt = reinterpret_cast<FT*>(w.W) + (size_t)b * n.nnzL;
       for (int t = gtid<NT>(); t < n.nnzL; t += NT) Wt[t] = wp<FT>(s)[t];
+      if (n.msm) {
+        double* Mt = w.M + (size_t)b * n.nT * top_ld(n.nT);
+        for (int t = gtid<NT>(); t < n.nT * top_ld(n.nT); t += NT) Mt[t] = s.Mg[t];
+      }
       for (int k = gtid<NT>(); k < n.L; k += NT) {
         const double q = s.q[k];
         w.P[(size_t)b * n.L + k] = s.P[k];
@@ -1895,8 +2003,12 @@ __device__ __forceinline__ void adjoint_one(const DevNet& n, const DevWork& w, c
   // kept state of scenario bf (several right-hand sides per scenario read the
   // same factor); right-hand sides, results and scratch are per b
   const int bf = (a.v0 + b) / (a.rhs_per > 1 ? a.rhs_per : 1);
-  s.Mg = w.M + (size_t)bf * n.nT * n.nT;  // terminal top-block inverse of the forward
+  double* Mt = w.M + (size_t)bf * n.nT * top_ld(n.nT);  // terminal top-block inverse of the forward
   if (!w.valid[bf]) return;  // uniform per group
+  if (n.msm)
+    for (int t = gtid<NT>(); t < n.nT * top_ld(n.nT); t += NT) s.Mg[t] = Mt[t];
+  else
+    s.Mg = Mt;
   const FT* Wt = reinterpret_cast<const FT*>(w.W) + (size_t)bf * n.nnzL;
   for (int t = gtid<NT>(); t < n.nnzL; t += NT) wp<FT>(s)[t] = Wt[t];
   for (int k = gtid<NT>(); k < n.L; k += NT) s.P[k] = w.P[(size_t)bf * n.L + k];
@@ -2200,7 +2312,7 @@ __device__ __forceinline__ void unrolled_one(const DevNet& n, const DevWork& w, 
   const int tid = gtid<NT>();
   s.q = w.lk + (size_t)b * 2 * n.L;
   s.Y = s.q + n.L;
-  s.Mg = w.M + (size_t)b * n.nT * n.nT;
+  if (!n.msm) s.Mg = w.M + (size_t)b * n.nT * top_ld(n.nT);
   const double* rrow = u.r + (long long)b * u.r_stride;
   const double* kerow = u.ke + (long long)b * u.ke_stride;
   const double* drow = u.d + (size_t)b * n.N;

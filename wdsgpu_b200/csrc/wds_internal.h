@@ -13,9 +13,12 @@ constexpr double kCSMALL = 1e-6;   // hydcoeffs.c CSMALL, dgga/solver.py:34
 constexpr double kCBIG = 1e8;      // dgga/solver.py:35
 constexpr double kBIG = 1e10;
 constexpr double kQZERO = 1e-6;
-// Columns of the dense top block at most (16 x 16 threads x 3 x 3 entries each
-// hold the block in registers while it is inverted).
+// Columns of the dense top block at most (six warps hold its six rows of 8 x 8
+// tiles in registers while it is inverted).
 constexpr int WDS_TOP_MAX = 48;
+// Row length of the stored inverse of the top block (even: rows are written in
+// 16-byte pieces).
+__host__ __device__ constexpr int top_ld(int nT) { return (nT + 1) & ~1; }
 
 // Device tables of one network.  Junction vectors are indexed by their
 // elimination index p (0..Nj-1); link ends are "end codes": p >= 0 for a
@@ -120,6 +123,8 @@ struct DevNet {
   // dense top block: levels [L0, nlev) = columns [cT, Nj), nT = Nj - cT
   // (nT = 0 and L0 = nlev when the network has none)
   int L0, cT, nT;
+  // the top block's inverse is part of the shared-memory state
+  int msm;
   // large network: slot-valued tables are 32-bit and stay in global memory
   // with the scenario state (one 256-thread CTA per scenario); otherwise the
   // 16-bit tables are staged into shared memory
@@ -141,7 +146,7 @@ struct DevWork {
   int8_t* act;    // [B][max(npcv,1)]
   double* scr;    // [B][nscr][Nj] scratch vectors
   double* lk;     // [B][2][L] link flows q and Y of the forward
-  double* M;      // [B][nT][nT] inverse of the top block's Schur complement
+  double* M;      // [B][nT][top_ld(nT)] inverse of the top block's Schur complement
   unsigned char* state;  // [B][state bytes] scenario state of large networks (else null)
   double* dpump;  // [B][3][npump] dhloss/d(speed, H0, R) of each pump at the terminal state
   double* dj;     // [B][Nj] the scenario's junction demands in elimination order

@@ -109,7 +109,7 @@ WorkOff work_layout(const wds::DevNet& d, int nscr, size_t B, size_t state_bytes
   o.W = take(B * d.nnzL * 8); o.P = take(B * d.L * 8); o.dr = take(B * d.L * 8);
   o.emh = take(B * d.Nj * 8); o.hge = take(B * d.Nj * 8); o.dke = take(B * d.Nj * 8);
   o.act = take(B * pc); o.scr = take(B * (size_t)nscr * d.Nj * 8); o.valid = take(B * 4);
-  o.lk = take(B * 2 * d.L * 8); o.M = take(B * (size_t)std::max(d.nT * d.nT, 1) * 8);
+  o.lk = take(B * 2 * d.L * 8); o.M = take(B * (size_t)std::max(d.nT * wds::top_ld(d.nT), 1) * 8);
   o.state = take(d.wide ? B * state_bytes : 0); o.pump = take(B * 3 * (size_t)d.npump * 8);
   o.dj = take(B * d.Nj * 8);
   o.bytes = bytes;
@@ -781,24 +781,31 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     plan->groups = 1;
     plan->smem_fwd = plan->smem_adj = 0;
   } else {
-    const size_t st = state_smem_bytes(d);
-    int best_g = 0, best_res = 0;
-    for (int g = 1; g <= 4; ++g) {
-      size_t sm = (size_t)d.stab_bytes + g * st;
-      if (sm > 227 * 1024) break;
-      int ctas = (int)((228 * 1024) / (sm + 1024));
-      ctas = std::min(ctas, 2048 / (256 * g));
-      if (ctas * g > best_res) { best_res = ctas * g; best_g = g; }
-    }
+    // the top block's inverse goes to shared memory where that leaves as many
+    // scenarios resident (a substitution reads it once: 4 k cycles from L2,
+    // 1.5 k from shared memory, one group per SM, 36 columns), else to L2
+    auto resident = [&](int msm, int g) {  // scenarios per SM; 0: does not fit
+      d.msm = msm;
+      const size_t sm = (size_t)d.stab_bytes + g * state_smem_bytes(d);
+      if (sm > 227 * 1024) return 0;
+      return g * std::min((int)((228 * 1024) / (sm + 1024)), 2048 / (256 * g));
+    };
+    int best_g = 0, best_res = 0, msm = 0;
+    for (int g = 1; g <= 4; ++g)
+      for (int m = d.nT > 0 ? 1 : 0; m >= 0; --m)
+        if (resident(m, g) > best_res) { best_res = resident(m, g); best_g = g; msm = m; }
     if (net->groups_per_cta > 0) {  // a tuned choice, if the state fits
-      if ((size_t)d.stab_bytes + net->groups_per_cta * st > 227 * 1024) {
+      if (resident(0, net->groups_per_cta) == 0) {
         cudaFree(plan->dtab);
         delete plan;
         return fail(WDS_E_ARG, "wds_plan: groups_per_cta " + std::to_string(net->groups_per_cta) +
                                    " exceeds shared memory for this network");
       }
       best_g = net->groups_per_cta;
+      msm = d.nT > 0 && resident(1, best_g) == resident(0, best_g) ? 1 : 0;
     }
+    d.msm = msm;
+    const size_t st = state_smem_bytes(d);
     plan->groups = best_g;
     plan->smem_fwd = best_g ? (size_t)d.stab_bytes + best_g * st : (size_t)d.stab_bytes + st;
     plan->smem_adj = plan->smem_fwd;
