@@ -991,32 +991,31 @@ __device__ void solve(const DevNet& n, const TB& T, const Sh& s, double* v) {
 }
 
 // x = A^{-1} rhs with `refine` refinement steps against the matrix-free A.
-// unit >= 0 means rhs = e_unit.  An unrefined solve whose x lies outside
-// shared memory (the Woodbury columns and refinement corrections in the
-// global workspace) runs in the shared temporary t and stores x once, so
-// that its substitution levels chain on shared-memory latency.
+// unit >= 0 means rhs = e_unit.  An x outside shared memory (the Woodbury
+// columns, refinement corrections and the unrolled adjoint in the global
+// workspace, the solution of a large network) is solved in the temporary t
+// when that lies inside, and stored, so that the substitutions chain on
+// shared-memory latency.
 template <int NT, class FT, class TB>
 __device__ void solve_refined(const DevNet& n, const TB& T, const Sh& s, const double* rhs,
                               int unit, double* x, double* t, int refine) {
   const int tid = gtid<NT>();
-  const bool via_t = refine == 0 && t != nullptr && !__isShared(x) && __isShared(t);
+  const bool via_t = !__isShared(x) && __isShared(t);
   double* v = via_t ? t : x;
   for (int p = tid; p < n.Nj; p += NT) v[p] = unit >= 0 ? (p == unit ? 1.0 : 0.0) : rhs[p];
   gsync<NT>();
-  solve<NT, FT>(n, T, s, v);
-  if (via_t) {
-    for (int p = tid; p < n.Nj; p += NT) x[p] = v[p];
-    gsync<NT>();
-    return;
-  }
-  for (int it = 0; it < refine; ++it) {
+  for (int it = 0;; ++it) {
+    solve<NT, FT>(n, T, s, v);
+    if (it > 0 || via_t) {
+      for (int p = tid; p < n.Nj; p += NT) x[p] = it > 0 ? x[p] + v[p] : v[p];
+      gsync<NT>();
+    }
+    if (it == refine) return;
+    v = t;
     for (int p = tid; p < n.Nj; p += NT) {
       const double b = unit >= 0 ? (p == unit ? 1.0 : 0.0) : rhs[p];
       t[p] = b - amul_node(n, T, s, p, x);
     }
-    gsync<NT>();
-    solve<NT, FT>(n, T, s, t);
-    for (int p = tid; p < n.Nj; p += NT) x[p] = x[p] + t[p];
     gsync<NT>();
   }
 }
@@ -1392,20 +1391,41 @@ __device__ void primal_solve(const DevNet& n, const TB& T, const Sh& s, double* 
   gsync<NT>();
 }
 
-__device__ __forceinline__ size_t al16(size_t x) { return (x + 15) / 16 * 16; }
-
 // doubles of V2: a node vector, or the top-block inversion's scratch
 __host__ __device__ inline int v2_len(const DevNet& n) {
   return n.nT > 0 && n.Nj < kTopScratch ? kTopScratch : n.Nj;
 }
 
-__device__ Sh carve(const DevNet& n, unsigned char* base) {
+__host__ __device__ __forceinline__ size_t al16(size_t x) { return (x + 15) / 16 * 16; }
+
+// The pieces of a scenario's state, in the order in which they claim shared
+// memory on the large-network layout: first what is small or always in use,
+// then the vector the substitutions run in, the solution, the factor, the
+// conductances and the rest.  take(bytes) places a piece and returns its
+// address (null when only sizes are wanted).
+template <class Take>
+__host__ __device__ __forceinline__ Sh place_state(const DevNet& n, Take&& take) {
   Sh s;
-  size_t o = 0;
-  auto take = [&](size_t bytes) { unsigned char* p = base + o; o = al16(o + bytes); return p; };
   s.q = nullptr;  // link flows and Y live in the global workspace (set by the kernel)
   s.Y = nullptr;
-  s.P = (double*)take(8ull * n.L);
+  s.red = (double*)take(8ull * 4 * 32);
+  s.wcnt = (int*)take(4ull * 32);
+  s.flag = (int*)take(16);      // [0] factor verdict, [1] error, [2] emitter count
+  s.err = s.flag + 1;
+  s.small = (double*)take(8ull * (4 * n.npcv * n.npcv + 5 * n.npcv + 8));
+  s.hf = (double*)take(8ull * (n.Nf > 0 ? n.Nf : 1));
+  s.xf = (double*)take(8ull * (n.nxf > 0 ? n.nxf : 1));
+  s.em_e = (double*)take(8ull * n.emcap);
+  s.em_ke = (double*)take(8ull * n.emcap);
+  s.em_emh = (double*)take(8ull * n.emcap);
+  // the solves' temporary; idle while the matrix is factored, so the top
+  // block's inversion works there
+  s.V2 = (double*)take(8ull * v2_len(n));
+  s.tb = s.V2;
+  // the top block's inverse, where it fits (else the kernel points it to the
+  // scenario's slice of the global workspace)
+  s.Mg = n.msm ? (double*)take(8ull * n.nT * top_ld(n.nT)) : nullptr;
+  s.V1 = (double*)take(8ull * n.Nj);
   if (n.fp32) {
     s.Wf = (float*)take(4ull * n.nnzL);
     s.W = nullptr;
@@ -1413,46 +1433,44 @@ __device__ Sh carve(const DevNet& n, unsigned char* base) {
     s.W = (double*)take(8ull * n.nnzL);
     s.Wf = nullptr;
   }
+  s.P = (double*)take(8ull * n.L);
   s.V0 = (double*)take(8ull * n.Nj);
-  s.V1 = (double*)take(8ull * n.Nj);
-  // the solves' temporary; idle while the matrix is factored, so the top
-  // block's inversion works there
-  s.V2 = (double*)take(8ull * v2_len(n));
-  s.tb = s.V2;
-  s.em_e = (double*)take(8ull * n.emcap);
-  s.em_ke = (double*)take(8ull * n.emcap);
-  s.em_emh = (double*)take(8ull * n.emcap);
-  s.hf = (double*)take(8ull * (n.Nf > 0 ? n.Nf : 1));
-  s.xf = (double*)take(8ull * (n.nxf > 0 ? n.nxf : 1));
-  s.red = (double*)take(8ull * 4 * 32);
-  s.small = (double*)take(8ull * (4 * n.npcv * n.npcv + 5 * n.npcv + 8));
-  s.eslot = (int16_t*)take(2ull * n.Nj);
-  // the top block's inverse, where it fits (else the kernel points it to the
-  // scenario's slice of the global workspace)
-  s.Mg = n.msm ? (double*)take(8ull * n.nT * top_ld(n.nT)) : nullptr;
-  s.wcnt = (int*)take(4ull * 32);
-  s.flag = (int*)take(16);      // [0] factor verdict, [1] error, [2] emitter count
-  s.err = s.flag + 1;
   s.S = (int8_t*)take(n.L);
+  s.eslot = (int16_t*)take(2ull * n.Nj);
   return s;
 }
 
-size_t smem_bytes(const DevNet& n) {
-  auto a16 = [](size_t x) { return (x + 15) / 16 * 16; };
+// The state at `base` (shared memory on the small-network layout).
+__device__ __forceinline__ Sh carve(const DevNet& n, unsigned char* base) {
   size_t o = 0;
-  o += a16(8ull * n.L);
-  o += a16((n.fp32 ? 4ull : 8ull) * n.nnzL);
-  o += 2 * a16(8ull * n.Nj) + a16(8ull * v2_len(n));
-  o += 3 * a16(8ull * n.emcap);
-  o += a16(8ull * (n.Nf > 0 ? n.Nf : 1));
-  o += a16(8ull * (n.nxf > 0 ? n.nxf : 1));
-  o += a16(8ull * 4 * 32);
-  o += a16(8ull * (4 * n.npcv * n.npcv + 5 * n.npcv + 8));
-  o += a16(2ull * n.Nj);
-  if (n.msm) o += a16(8ull * n.nT * top_ld(n.nT));
-  o += a16(4ull * 32);
-  o += a16(16);
-  o += a16(n.L);
+  return place_state(n, [&](size_t bytes) {
+    unsigned char* p = base + o;
+    o += al16(bytes);
+    return p;
+  });
+}
+
+// The state of the large-network layout: each piece in the n.sm_state bytes
+// of shared memory at `sm` while they last, else in the scenario's slice of
+// the global workspace.
+__device__ __forceinline__ Sh carve_split(const DevNet& n, unsigned char* sm,
+                                          unsigned char* base) {
+  size_t os = 0, og = 0;
+  return place_state(n, [&](size_t bytes) {
+    const bool in = os + al16(bytes) <= (size_t)n.sm_state;
+    unsigned char* p = in ? sm + os : base + og;
+    (in ? os : og) += al16(bytes);
+    return p;
+  });
+}
+
+// Bytes of a scenario's state.
+size_t smem_bytes(const DevNet& n) {
+  size_t o = 0;
+  place_state(n, [&](size_t bytes) -> unsigned char* {
+    o += al16(bytes);
+    return nullptr;
+  });
   return o;
 }
 
@@ -1533,7 +1551,7 @@ __device__ __forceinline__ void cta_rounds(const DevNet& n, const DevWork& w, in
     if (r > 0) gsync<NT>();  // the previous scenario's last reads of the group state
     Sh s;
     if constexpr (TB::kWide)
-      s = carve(n, w.state + (size_t)b * state_bytes);
+      s = carve_split(n, smem_raw, w.state + (size_t)b * state_bytes);
     else
       s = carve(n, smem_raw + n.stab_bytes + (size_t)g * state_bytes);
     one(T, s, b);
@@ -2479,34 +2497,34 @@ __global__ void __launch_bounds__(NT * GR, 1) k_adjoint(DevNet n, DevWork w, Adj
   adjoint_body<NT, TB, FT>(n, w, a, state_bytes, blockIdx.x, gridDim.x, GR);
 }
 
-// Several plans (networks of different sizes) in one launch: CTAs
-// [job.cta0, next job's cta0) run the job's plan, with 3 groups of 256
-// threads each (a plan that fits fewer groups in shared memory leaves the
-// others idle; large-network plans run 3 scenarios per CTA from global memory).
+// Several plans (networks of different sizes) in one launch of 1024-thread
+// CTAs: CTAs [job.cta0, next job's cta0) run the job's plan, a small network
+// with J.groups groups of 256 threads (the others idle), a large one with one
+// scenario per CTA.
 template <class FT>
-__global__ void __launch_bounds__(768, 1) k_forward_multi(const __grid_constant__ FwdJobs jobs) {
+__global__ void __launch_bounds__(kWideThreads, 1)
+    k_forward_multi(const __grid_constant__ FwdJobs jobs) {
   int p = 0;
   while (p + 1 < jobs.n && (int)blockIdx.x >= jobs.j[p + 1].cta0) ++p;
   const FwdJob& J = jobs.j[p];
+  const int ctas = (J.a.B + J.groups - 1) / J.groups, c = blockIdx.x - J.cta0;
   if (J.n.wide)
-    forward_body<256, LTab, FT>(J.n, J.w, J.a, J.state_bytes, blockIdx.x - J.cta0,
-                                (J.a.B + J.groups - 1) / J.groups, J.groups);
+    forward_body<kWideThreads, LTab, FT>(J.n, J.w, J.a, J.state_bytes, c, ctas, 1);
   else
-    forward_body<256, STab, FT>(J.n, J.w, J.a, J.state_bytes, blockIdx.x - J.cta0,
-                                (J.a.B + J.groups - 1) / J.groups, J.groups);
+    forward_body<256, STab, FT>(J.n, J.w, J.a, J.state_bytes, c, ctas, J.groups);
 }
 
 template <class FT>
-__global__ void __launch_bounds__(768, 1) k_adjoint_multi(const __grid_constant__ AdjJobs jobs) {
+__global__ void __launch_bounds__(kWideThreads, 1)
+    k_adjoint_multi(const __grid_constant__ AdjJobs jobs) {
   int p = 0;
   while (p + 1 < jobs.n && (int)blockIdx.x >= jobs.j[p + 1].cta0) ++p;
   const AdjJob& J = jobs.j[p];
+  const int ctas = (J.a.B + J.groups - 1) / J.groups, c = blockIdx.x - J.cta0;
   if (J.n.wide)
-    adjoint_body<256, LTab, FT>(J.n, J.w, J.a, J.state_bytes, blockIdx.x - J.cta0,
-                                (J.a.B + J.groups - 1) / J.groups, J.groups);
+    adjoint_body<kWideThreads, LTab, FT>(J.n, J.w, J.a, J.state_bytes, c, ctas, 1);
   else
-    adjoint_body<256, STab, FT>(J.n, J.w, J.a, J.state_bytes, blockIdx.x - J.cta0,
-                                (J.a.B + J.groups - 1) / J.groups, J.groups);
+    adjoint_body<256, STab, FT>(J.n, J.w, J.a, J.state_bytes, c, ctas, J.groups);
 }
 
 }  // namespace

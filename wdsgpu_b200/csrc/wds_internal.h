@@ -16,6 +16,10 @@ constexpr double kQZERO = 1e-6;
 // Columns of the dense top block at most (six warps hold its six rows of 8 x 8
 // tiles in registers while it is inverted).
 constexpr int WDS_TOP_MAX = 48;
+// Threads of a scenario of a large network (one CTA): most of its time goes to
+// the passes over links, junctions and wide levels, which 256 threads cover in
+// four times as many steps, and no second scenario fits beside it.
+constexpr int kWideThreads = 1024;
 // Row length of the stored inverse of the top block (even: rows are written in
 // 16-byte pieces).
 __host__ __device__ constexpr int top_ld(int nT) { return (nT + 1) & ~1; }
@@ -123,8 +127,11 @@ struct DevNet {
   // dense top block: levels [L0, nlev) = columns [cT, Nj), nT = Nj - cT
   // (nT = 0 and L0 = nlev when the network has none)
   int L0, cT, nT;
-  // the top block's inverse is part of the shared-memory state
+  // the top block's inverse is part of the state placed by place_state
   int msm;
+  // large networks: bytes of shared memory that hold the first pieces of the
+  // scenario's state
+  int sm_state;
   // large network: slot-valued tables are 32-bit and stay in global memory
   // with the scenario state (one 256-thread CTA per scenario); otherwise the
   // 16-bit tables are staged into shared memory

@@ -3,7 +3,7 @@
 
 namespace wds {
 const void* WDS_KSEL(forward_kernel)(int wide, int groups) {
-  if (wide) return (const void*)k_forward<256, 1, LTab, KFT>;
+  if (wide) return (const void*)k_forward<kWideThreads, 1, LTab, KFT>;
   switch (groups) {
     case 1: return (const void*)k_forward<256, 1, STab, KFT>;
     case 2: return (const void*)k_forward<256, 2, STab, KFT>;

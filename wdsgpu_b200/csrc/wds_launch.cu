@@ -33,8 +33,9 @@ size_t multi_smem(const Jobs& jobs) {
   size_t smem = 0;
   for (int p = 0; p < jobs.n; ++p) {
     const auto& J = jobs.j[p];
-    if (!J.n.wide)
-      smem = std::max(smem, (size_t)J.n.stab_bytes + (size_t)J.groups * (size_t)J.state_bytes);
+    smem = std::max(smem, J.n.wide ? (size_t)J.n.sm_state
+                                   : (size_t)J.n.stab_bytes +
+                                         (size_t)J.groups * (size_t)J.state_bytes);
   }
   return smem;
 }
@@ -45,20 +46,21 @@ template <class Args>
 int launch_single(const void* kern, const DevNet& n, const DevWork& w, const Args& a, int B,
                   int groups, void* stream, const char* who, std::string* err) {
   int st = (int)smem_bytes(n);
-  const size_t smem = n.wide ? 0 : (size_t)n.stab_bytes + (size_t)groups * st;
+  const size_t smem = n.wide ? (size_t)n.sm_state : (size_t)n.stab_bytes + (size_t)groups * st;
+  const int threads = n.wide ? kWideThreads : 256 * groups;
   cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (ce != cudaSuccess) {
     *err = std::string(who) + ": " + cudaGetErrorString(ce);
     return WDS_E_CUDA;
   }
   int grid = 1;
-  ce = persistent_grid(kern, 256 * groups, smem, B, &grid);
+  ce = persistent_grid(kern, threads, smem, B, &grid);
   if (ce == cudaSuccess) {
     DevNet n_ = n;
     DevWork w_ = w;
     Args a_ = a;
     void* args[] = {&n_, &w_, &a_, &st};
-    ce = cudaLaunchKernel(kern, dim3(grid), dim3(256 * groups), args, smem, (cudaStream_t)stream);
+    ce = cudaLaunchKernel(kern, dim3(grid), dim3(threads), args, smem, (cudaStream_t)stream);
   }
   if (ce != cudaSuccess) {
     *err = std::string(who) + " launch: " + cudaGetErrorString(ce);
@@ -74,7 +76,7 @@ int launch_jobs(const void* kern, Jobs& jobs, int ctas, void* stream, const char
   cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (ce == cudaSuccess && ctas > 0) {
     void* args[] = {&jobs};
-    ce = cudaLaunchKernel(kern, dim3(ctas), dim3(768), args, smem, (cudaStream_t)stream);
+    ce = cudaLaunchKernel(kern, dim3(ctas), dim3(kWideThreads), args, smem, (cudaStream_t)stream);
   }
   if (ce != cudaSuccess) {
     *err = std::string(who) + ": " + cudaGetErrorString(ce);

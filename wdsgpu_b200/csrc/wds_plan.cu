@@ -777,9 +777,13 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
   plan->threads = 256;
   // scenario groups per CTA: the count that keeps the most scenarios resident
   // per SM (228 KB of shared memory per SM, 1 KB reserved per CTA)
-  if (d.wide) {  // large network: one 256-thread CTA per scenario, state in global memory
+  if (d.wide) {
+    // large network: one CTA per scenario, tables in global memory; the state
+    // as far as it fits in shared memory, the rest in global memory
     plan->groups = 1;
     plan->smem_fwd = plan->smem_adj = 0;
+    d.msm = d.nT > 0 ? 1 : 0;
+    d.sm_state = (int)std::min<size_t>(state_smem_bytes(d), 227 * 1024);
   } else {
     // the top block's inverse goes to shared memory where that leaves as many
     // scenarios resident (a substitution reads it once: 4 k cycles from L2,
@@ -821,7 +825,7 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
   DevWork& w = plan->dw;
   // heads, rp, res, sx, 2p Woodbury columns, 2p+1 per-warp temporaries
   const int nscr = 5 + 4 * std::max(npcv, 1);
-  const WorkOff wo = work_layout(d, nscr, (size_t)max_batch, state_bytes);
+  const WorkOff wo = work_layout(d, nscr, (size_t)max_batch, state_smem_bytes(d));
   const size_t bytes = wo.bytes;
   if (cudaMalloc(&plan->dwork, bytes) != cudaSuccess) {
     cudaFree(plan->dtab);
@@ -972,7 +976,7 @@ extern "C" int wds_forward_multi(int32_t nplans, WdsPlan* const* plans, const in
     FwdJob& J = jobs.j[p];
     J.n = plan->dn;
     J.w = plan->dw;
-    J.groups = plan->dn.wide ? 3 : std::min(3, plan->groups);
+    J.groups = plan->groups;
     FwdArgs& a = J.a;
     a.B = batch[p]; a.hacc = o->accuracy; a.max_iter = o->max_iter;
     a.sm = o->status_machine ? 1 : 0; a.refine = o->refine; a.polish = o->polish_steps;
@@ -1013,7 +1017,7 @@ extern "C" int wds_adjoint_multi(int32_t nplans, WdsPlan* const* plans, const in
     AdjJob& J = jobs.j[p];
     J.n = plan->dn;
     J.w = plan->dw;
-    J.groups = plan->dn.wide ? 3 : std::min(3, plan->groups);
+    J.groups = plan->groups;
     J.a = AdjArgs{batch[p], x.gH, x.gQ, x.gE, x.gd, x.grh, x.gke, x.gr};
   }
   std::string err;
