@@ -299,6 +299,16 @@ int wds_adjoint_rhs(WdsPlan* plan, int32_t batch, int32_t rhs_per, int32_t first
                     const double* gH, const double* gQ, const double* gE, double* gd,
                     double* grh, double* gke, double* gr, void* stream);
 
+/* Resistance gradients of unit head adjoints on the terminal factors of the
+ * last implicit wds_forward: row b is right-hand side number first + b of
+ * scenario (first + b) / rhs_per, the head of node nodes[(first + b) % rhs_per]
+ * (device array [rhs_per]), and gr [rows][L] receives d head / d r.  Any number
+ * of rows in one launch (their scratch is by resident scenario, allocated by
+ * the first call that needs it and kept by the plan).  As wds_adjoint_rhs with
+ * a unit gH row and zero gQ, gE. */
+int wds_sensitivity(WdsPlan* plan, int32_t rows, int32_t rhs_per, int32_t first,
+                    const int32_t* nodes, double* gr, void* stream);
+
 /* Device arrays of one plan in a multi-plan call (shapes as in wds_forward /
  * wds_adjoint). */
 typedef struct WdsForwardIO {

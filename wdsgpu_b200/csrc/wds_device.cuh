@@ -1531,7 +1531,7 @@ __device__ bool build_emitters(const DevNet& n, const Sh& s, const double* val, 
 template <int NT, class TB, class One>
 __device__ __forceinline__ void cta_rounds(const DevNet& n, const DevWork& w, int B,
                                            int state_bytes, int blk, int nblk, int groups,
-                                           One&& one) {
+                                           One&& one, bool by_slot = false) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int g = threadIdx.x / NT;
   TB T;
@@ -1551,7 +1551,8 @@ __device__ __forceinline__ void cta_rounds(const DevNet& n, const DevWork& w, in
     if (r > 0) gsync<NT>();  // the previous scenario's last reads of the group state
     Sh s;
     if constexpr (TB::kWide)
-      s = carve_split(n, smem_raw, w.state + (size_t)b * state_bytes);
+      s = carve_split(n, smem_raw,
+                      w.state + (size_t)(by_slot ? blk * groups + g : b) * state_bytes);
     else
       s = carve(n, smem_raw + n.stab_bytes + (size_t)g * state_bytes);
     one(T, s, b);
@@ -2015,9 +2016,11 @@ __device__ __forceinline__ void forward_body(const DevNet& n, const DevWork& w, 
 // Node adjoint with constraint rows (autodiff.py:1107-1154) and the
 // theta contraction (autodiff.py:1246-1312).
 // Adjoint of right-hand side b by one scenario group.
+// With a.unit the right-hand side is the unit head adjoint of one node and only
+// the resistance gradient is wanted.  `slot` numbers the scratch vectors.
 template <int NT, class TB, class FT>
 __device__ __forceinline__ void adjoint_one(const DevNet& n, const DevWork& w, const AdjArgs& a,
-                                            const TB& T, Sh s, int b) {
+                                            const TB& T, Sh s, int b, int slot) {
   // kept state of scenario bf (several right-hand sides per scenario read the
   // same factor); right-hand sides, results and scratch are per b
   const int bf = (a.v0 + b) / (a.rhs_per > 1 ? a.rhs_per : 1);
@@ -2044,11 +2047,15 @@ __device__ __forceinline__ void adjoint_one(const DevNet& n, const DevWork& w, c
     if (es >= 0) s.em_emh[es] = w.emh[(size_t)bf * n.Nj + p];
   }
   gsync<NT>();
-  const double* gH = a.gH + (size_t)b * n.N;
-  const double* gQ = a.gQ + (size_t)b * n.L;
-  const double* gE = a.gE + (size_t)b * n.N;
+  const bool unit = a.unit != nullptr;
+  const int unode = unit ? a.unit[(a.v0 + b) % a.rhs_per] : -1;
+  const double* gH = unit ? nullptr : a.gH + (size_t)b * n.N;
+  const double* gQ = unit ? nullptr : a.gQ + (size_t)b * n.L;
+  const double* gE = unit ? nullptr : a.gE + (size_t)b * n.N;
   // r = B^T P gQ - em gE / hge - gH
-  for (int p = gtid<NT>(); p < n.Nj; p += NT) {
+  if (unit)
+    for (int p = gtid<NT>(); p < n.Nj; p += NT) s.V0[p] = n.jnode[p] == unode ? -1.0 : 0.0;
+  else for (int p = gtid<NT>(); p < n.Nj; p += NT) {
     const int a0 = T.inc_ptr[p], m = T.inc_split[p], z = T.inc_ptr[p + 1];
     double acc = 0.0;
     for (int e = m; e < z; ++e) {
@@ -2072,7 +2079,7 @@ __device__ __forceinline__ void adjoint_one(const DevNet& n, const DevWork& w, c
     solve_refined<NT, FT>(n, T, s, s.V0, -1, lam, t, 2);
   } else {
     const int p = n.npcv;
-    double* scr = w.scr + (size_t)b * w.nscr * n.Nj;
+    double* scr = w.scr + (size_t)slot * w.nscr * n.Nj;
     double* r2 = scr;
     double* res = r2 + n.Nj;
     double* sx = res + n.Nj;
@@ -2088,7 +2095,7 @@ __device__ __forceinline__ void adjoint_one(const DevNet& n, const DevWork& w, c
       for (int i = 0; i < p; ++i)
         // row jc: lam[n2] - lam[n1] = gQ of the free valve flow, i.e.
         // lam[jc] - lam[jo] = sgn gQ (PRV jc = n2, PSV jc = n1)
-        if (actf[i] != 0.0) r2[n.pcv_jc[i]] = n.pcv_sgn[i] * gQ[n.pcv_link[i]];
+        if (actf[i] != 0.0) r2[n.pcv_jc[i]] = unit ? 0.0 : n.pcv_sgn[i] * gQ[n.pcv_link[i]];
     gsync<NT>();
     // unrefined solves: the two outer refinement steps below contract their error
     solve_refined<NT, FT>(n, T, s, r2, -1, lam, t, 0);
@@ -2139,6 +2146,15 @@ __device__ __forceinline__ void adjoint_one(const DevNet& n, const DevWork& w, c
     }
   }
   // theta contraction
+  if (unit) {
+    const double* dr = w.dr + (size_t)bf * n.L;
+    double* gr = a.gr + (size_t)b * n.L;
+    for (int k = gtid<NT>(); k < n.L; k += NT) {
+      const double l1 = junc_of(T.e1[k], lam), l2 = junc_of(T.e2[k], lam);
+      gr[k] = s.P[k] * (l2 - l1) * dr[k];
+    }
+    return;
+  }
   double* gd = a.gd + (size_t)b * n.N;
   double* gke = a.gke + (size_t)b * n.N;
   double* grh = a.grh + (size_t)b * n.N;
@@ -2197,9 +2213,10 @@ __device__ __forceinline__ void adjoint_one(const DevNet& n, const DevWork& w, c
 template <int NT, class TB, class FT>
 __device__ __forceinline__ void adjoint_body(const DevNet& n, const DevWork& w, const AdjArgs& a,
                                              int state_bytes, int blk, int nblk, int groups) {
+  const int slot = blk * groups + (int)(threadIdx.x / NT);
   cta_rounds<NT, TB>(n, w, a.B, state_bytes, blk, nblk, groups, [&](const TB& T, Sh s, int b) {
-    adjoint_one<NT, TB, FT>(n, w, a, T, s, b);
-  });
+    adjoint_one<NT, TB, FT>(n, w, a, T, s, b, a.by_slot ? slot : b);
+  }, a.by_slot != 0);
 }
 
 // ---------------------------------------------------------------- unrolled-K reverse

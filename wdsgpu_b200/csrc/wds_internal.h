@@ -210,6 +210,12 @@ struct AdjArgs {
   // (v0 + b) / rhs_per; 0 or 1 means one right-hand side per scenario
   int rhs_per = 1;
   int v0 = 0;
+  // unit head adjoints: node of right-hand side v at unit[v % rhs_per]; only
+  // gr is written (null: the arrays above)
+  const int* unit = nullptr;
+  // scratch vectors and global state by resident scenario group instead of by
+  // row (more rows than the workspace holds scenarios)
+  int by_slot = 0;
 };
 
 // Host-side symbolic data kept in the plan (for inspection and tests).
@@ -247,6 +253,8 @@ int launch_forward(const DevNet& n, const DevWork& w, const FwdArgs& a, int grou
 int launch_adjoint(const DevNet& n, const DevWork& w, const AdjArgs& a, int groups,
                    void* stream, std::string* err);
 size_t state_smem_bytes(const DevNet& n);
+// CTAs of a launch of the adjoint over `rows` rows (-1: a CUDA error in *err)
+int adjoint_grid(const DevNet& n, int groups, int rows, std::string* err);
 
 // One plan's share of a multi-plan launch.  `groups` is the number of
 // scenario groups (256 threads each) per 768-thread CTA; state_bytes and cta0

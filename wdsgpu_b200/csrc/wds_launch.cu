@@ -40,14 +40,21 @@ size_t multi_smem(const Jobs& jobs) {
   return smem;
 }
 
+// Shared memory and threads of a single-plan launch of `groups` scenario groups
+// per CTA (large networks: one).
+size_t launch_smem(const DevNet& n, int groups) {
+  return n.wide ? (size_t)n.sm_state : (size_t)n.stab_bytes + (size_t)groups * smem_bytes(n);
+}
+int launch_threads(const DevNet& n, int groups) { return n.wide ? kWideThreads : 256 * groups; }
+
 // One persistent single-plan launch of `kern` (arguments: DevNet, DevWork,
 // the call's argument block, the per-group state bytes).
 template <class Args>
 int launch_single(const void* kern, const DevNet& n, const DevWork& w, const Args& a, int B,
                   int groups, void* stream, const char* who, std::string* err) {
   int st = (int)smem_bytes(n);
-  const size_t smem = n.wide ? (size_t)n.sm_state : (size_t)n.stab_bytes + (size_t)groups * st;
-  const int threads = n.wide ? kWideThreads : 256 * groups;
+  const size_t smem = launch_smem(n, groups);
+  const int threads = launch_threads(n, groups);
   cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (ce != cudaSuccess) {
     *err = std::string(who) + ": " + cudaGetErrorString(ce);
@@ -134,6 +141,19 @@ int launch_unrolled(const DevNet& n, const DevWork& w, const UnrollArgs& u, int 
   const int groups = n.wide ? 1 : std::min(plan_groups, 3);  // at most 3 groups per CTA
   const void* kern = n.fp32 ? unrolled_kernel_f32(n.wide, groups) : unrolled_kernel_f64(n.wide, groups);
   return launch_single(kern, n, w, u, u.B, groups, stream, "wds_unrolled_adjoint", err);
+}
+
+int adjoint_grid(const DevNet& n, int groups, int rows, std::string* err) {
+  const void* kern = n.fp32 ? adjoint_kernel_f32(n.wide, groups) : adjoint_kernel_f64(n.wide, groups);
+  const size_t smem = launch_smem(n, groups);
+  int grid = 1;
+  cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (ce == cudaSuccess) ce = persistent_grid(kern, launch_threads(n, groups), smem, rows, &grid);
+  if (ce != cudaSuccess) {
+    *err = std::string("wds_sensitivity: ") + cudaGetErrorString(ce);
+    return -1;
+  }
+  return grid;
 }
 
 int launch_adjoint(const DevNet& n, const DevWork& w, const AdjArgs& a, int groups,

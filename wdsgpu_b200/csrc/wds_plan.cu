@@ -139,6 +139,10 @@ struct WdsPlan {
   wds::HostSym sym;
   void* dtab = nullptr;
   void* dwork = nullptr;
+  // scratch of wds_sensitivity by resident scenario group (allocated on first
+  // use, grown when a call has more resident groups)
+  void* drows = nullptr;
+  int rows_slots = 0;
   int max_batch = 0;
   int threads = 256;
   int groups = 1;
@@ -950,6 +954,50 @@ extern "C" int wds_adjoint_rhs(WdsPlan* plan, int32_t batch, int32_t rhs_per, in
   return WDS_OK;
 }
 
+extern "C" int wds_sensitivity(WdsPlan* plan, int32_t rows, int32_t rhs_per, int32_t first,
+                               const int32_t* nodes, double* gr, void* stream) {
+  using namespace wds;
+  if (!plan || rows <= 0 || rhs_per <= 0 || first < 0 || !nodes || !gr)
+    return fail(WDS_E_ARG, "wds_sensitivity: bad argument");
+  if (!plan->have_state)
+    return fail(WDS_E_STATE, "wds_sensitivity: no implicit forward to differentiate");
+  if ((int64_t)first + rows - 1 >= (int64_t)plan->state_batch * rhs_per)
+    return fail(WDS_E_ARG, "wds_sensitivity: rows beyond the kept scenarios");
+  std::string err;
+  const DevNet& d = plan->dn;
+  DevWork w = plan->dw;
+  AdjArgs a{};
+  a.B = rows;
+  a.gr = gr;
+  a.rhs_per = rhs_per;
+  a.v0 = first;
+  a.unit = nodes;
+  a.by_slot = 1;
+  // scratch vectors are read with ACTIVE valves only, the state in global
+  // memory only when it exceeds shared memory
+  const size_t st = state_smem_bytes(d);
+  const size_t scr = d.npcv > 0 ? ((size_t)w.nscr * d.Nj * 8 + 255) / 256 * 256 : 0;
+  const size_t glob = d.wide && st > (size_t)d.sm_state ? (st + 255) / 256 * 256 : 0;
+  if (scr + glob > 0) {
+    const int grid = adjoint_grid(d, plan->groups, rows, &err);
+    if (grid < 0) return fail(WDS_E_CUDA, err);
+    const int slots = grid * plan->groups;
+    if (slots > plan->rows_slots) {
+      if (plan->drows) cudaFree(plan->drows);
+      plan->drows = nullptr;
+      plan->rows_slots = 0;
+      if (cudaMalloc(&plan->drows, (size_t)slots * (scr + glob)) != cudaSuccess)
+        return fail(WDS_E_NOMEM, "wds_sensitivity: cudaMalloc of the rows' scratch failed");
+      plan->rows_slots = slots;
+    }
+    if (scr) w.scr = (double*)plan->drows;
+    if (glob) w.state = (unsigned char*)plan->drows + (size_t)plan->rows_slots * scr;
+  }
+  const int rc = launch_adjoint(d, w, a, plan->groups, stream, &err);
+  if (rc != WDS_OK) return fail(rc, err);
+  return WDS_OK;
+}
+
 extern "C" int wds_forward_multi(int32_t nplans, WdsPlan* const* plans, const int32_t* batch,
                                  const WdsForwardOpts* opts, const WdsForwardIO* io,
                                  void* stream) {
@@ -1096,6 +1144,7 @@ extern "C" int wds_free(WdsPlan* plan) {
   if (!plan) return WDS_OK;
   if (plan->dtab) cudaFree(plan->dtab);
   if (plan->dwork) cudaFree(plan->dwork);
+  if (plan->drows) cudaFree(plan->drows);
   delete plan;
   return WDS_OK;
 }

@@ -3,8 +3,8 @@
 Mirrors dgga/sensitivity.py:59-145 (`sensitivity_matrix`).  The reference
 factorises the Jacobian once per frame and solves m sensor columns with it;
 here one implicit forward keeps each scenario's terminal factor on the GPU and
-`wds_adjoint_rhs` runs the m adjoints of every frame on it (row v = frame
-v // m, sensor v % m), in launches of up to the plan's capacity.  No new
+`wds_sensitivity` runs the m adjoints of every frame on it (row v = frame
+v // m, sensor v % m) in one launch.  No new
 factorisation.  dp_i/dr_k = dH_i/dr_k (p = H - El); the C chain factor is
 dr/dC = -Hexp r / C on H-W pipes and 0 elsewhere (dgga/calib.py dr_dC).
 """
@@ -22,6 +22,7 @@ from .solver import GGASolver, _check_info_flags, _not_pd_hint
 __all__ = ["sensitivity_matrix", "dr_dC_chain"]
 
 _PIPE_KINDS = (0, 1)      # CVPIPE, PIPE
+_CHUNK_BYTES = 256 << 20  # gradients of one launch
 
 
 def dr_dC_chain(solver: GGASolver, r_hw=None):
@@ -79,30 +80,25 @@ def sensitivity_matrix(solver, demand, res_head, r_hw, sensor_nodes, wrt="C", fr
     dev = s.device
     fr = list(range(B)) if frames is None else [int(b) for b in frames]
     rows = B * m
-    cap = plan.max_batch
-    S = np.empty((rows, s.L))
-    sens_t = torch.as_tensor(sensors, device=dev)
+    sens_t = torch.as_tensor(sensors.astype(np.int32), device=dev)
+    chain = torch.as_tensor(dr_dC_chain(s, r_hw), device=dev) if wrt == "C" else None
     cur = torch.cuda.current_stream(dev)
     t1 = perf_counter()
-    for v0 in range(0, rows, cap):
-        nb = min(cap, rows - v0)
-        gH = torch.zeros(nb, s.N, dtype=torch.float64, device=dev)
-        v = torch.arange(v0, v0 + nb, device=dev)
-        gH[torch.arange(nb, device=dev), sens_t[v % m]] = 1.0
-        gQ = torch.zeros(nb, s.L, dtype=torch.float64, device=dev)
-        gE = torch.zeros(nb, s.N, dtype=torch.float64, device=dev)
-        gd = torch.empty(nb, s.N, dtype=torch.float64, device=dev)
-        grh, gke = torch.empty_like(gd), torch.empty_like(gd)
+    parts = []
+    step = max(1, _CHUNK_BYTES // (8 * s.L))   # rows whose gradients are on the device at once
+    for v0 in range(0, rows, step):
+        nb = min(step, rows - v0)
         gr = torch.empty(nb, s.L, dtype=torch.float64, device=dev)
-        _lib.check(plan.lib.wds_adjoint_rhs(
-            plan.handle, nb, m, v0, gH.data_ptr(), gQ.data_ptr(), gE.data_ptr(), gd.data_ptr(),
-            grh.data_ptr(), gke.data_ptr(), gr.data_ptr(), ctypes.c_void_p(cur.cuda_stream)),
-            "wds_adjoint_rhs")
-        S[v0:v0 + nb] = gr.cpu().numpy()
+        _lib.check(plan.lib.wds_sensitivity(
+            plan.handle, nb, m, v0, sens_t.data_ptr(), gr.data_ptr(),
+            ctypes.c_void_p(cur.cuda_stream)), "wds_sensitivity")
+        if chain is not None:
+            gr.mul_(chain)
+        parts.append(gr.cpu().numpy())
+    S = parts[0] if len(parts) == 1 else np.concatenate(parts or [np.empty((0, s.L))])
     t_adj = perf_counter() - t1
-    if wrt == "C":
-        S = S * dr_dC_chain(s, r_hw if r_hw is not None else None)[None, :]
-    S = S.reshape(B, m, s.L)[fr].reshape(len(fr) * m, s.L)
+    if frames is not None:
+        S = S.reshape(B, m, s.L)[fr].reshape(len(fr) * m, s.L)
     if return_info:
         return S, dict(frames=fr, sensors=sensors, n_factorizations=0, n_rhs=len(fr) * m,
                        t_forward=t_forward, t_adjoint=t_adj)
