@@ -193,11 +193,15 @@ class ImplicitGGASolveSM100(torch.autograd.Function):
         if ke_t.shape[0] == 1 and B > 1:
             ke_t = ke_t.contiguous()
         th_in = (speed, pump_h0, pump_r)
-        pumps = s.pump_rows(B, *th_in)
+        later = []
+        pumps = s.pump_rows(B, *th_in, later=later)
         o = s.run(d, rh, ke_t, r_t, B, int(max_iter), float(accuracy), sm, int(polish_steps),
                   pumps=pumps)
         info = o["info"]
-        if bool((info != 0).any()):   # one host sync when every scenario converged
+        host_info = info.cpu().numpy()   # the host's one wait when every scenario converged
+        for check in later:
+            check()
+        if host_info.any():
             from .solver import _check_info_flags
             _check_info_flags(s, info)
             bad = torch.nonzero(info != 0).flatten().tolist()
@@ -346,7 +350,7 @@ class UnrolledSM100(torch.autograd.Function):
         o = s.run(d, rh, ke_t, r_t, B, int(K), 1e-12, False, -1, refine=2, refine_band=0.0,
                   record=rec, q0=q0, e0=e0, S0=S0)
         info = o["info"]
-        if bool((info != 0).any()):
+        if info.cpu().numpy().any():
             from .solver import _check_info_flags
             _check_info_flags(s, info)
             bad = torch.nonzero(info != 0).flatten().tolist()

@@ -108,8 +108,8 @@ class _Tanks:
 def _step_forward(s, d, rh, ke, r, B, max_iter, acc, polish, q0, e0, S0=None):
     o = s.run(d, rh, ke, r, B, max_iter, acc, True, polish, q0=q0, e0=e0, S0=S0)
     info = o["info"]
-    _check_info_flags(s, info)
-    if bool((info != 0).any()):
+    if info.cpu().numpy().any():
+        _check_info_flags(s, info)
         bad = torch.nonzero(info != 0).flatten().tolist()
         if bool((info & _lib.INFO_NOT_PD).any()):
             raise RuntimeError("eps: the node matrix of scenarios %s is not positive definite%s"

@@ -94,11 +94,12 @@ def solve_multi(solvers, demands, res_heads, kes=None, r_hws=None, accuracy=None
     res = []
     for s, o in zip(solvers, outs):
         info = o["info"]
-        _check_info_flags(s, info)
-        bad = torch.nonzero(info & _lib.INFO_NOT_PD).flatten()
-        if bad.numel():
-            raise RuntimeError("batched LDL^T failed: the node matrix of scenarios %s is not "
-                               "positive definite%s" % (bad.tolist(), _not_pd_hint(s)))
+        if info.cpu().numpy().any():
+            _check_info_flags(s, info)
+            bad = torch.nonzero(info & _lib.INFO_NOT_PD).flatten()
+            if bad.numel():
+                raise RuntimeError("batched LDL^T failed: the node matrix of scenarios %s is not "
+                                   "positive definite%s" % (bad.tolist(), _not_pd_hint(s)))
         r = dict(head_ft=o["head"], flow_cfs=o["flow"], emitter_cfs=o["emit"],
                  iters=o["iters"].to(torch.int64), relerr=o["relerr"], converged=(info == 0))
         if status_machine:
@@ -122,8 +123,8 @@ class ImplicitMultiSM100(torch.autograd.Function):
         res, clamps = [], []
         for s, o in zip(solvers, outs):
             info = o["info"]
-            _check_info_flags(s, info)
-            if bool((info != 0).any()):
+            if info.cpu().numpy().any():
+                _check_info_flags(s, info)
                 bad = torch.nonzero(info != 0).flatten().tolist()
                 if bool((info & _lib.INFO_NOT_PD).any()):
                     raise RuntimeError("implicit_solve_multi: the node matrix of scenarios %s "

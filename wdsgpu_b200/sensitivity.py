@@ -67,8 +67,8 @@ def sensitivity_matrix(solver, demand, res_head, r_hw, sensor_nodes, wrt="C", fr
     o = s.run(d, rh, ke_t.contiguous(), r_t.contiguous(), B, int(max_iter), float(accuracy),
               True, int(polish_steps), pumps=pumps)
     info_v = o["info"]
-    _check_info_flags(s, info_v)
-    if bool((info_v != 0).any()):
+    if info_v.cpu().numpy().any():
+        _check_info_flags(s, info_v)
         badb = torch.nonzero(info_v != 0).flatten().tolist()
         if bool((info_v & _lib.INFO_NOT_PD).any()):
             raise RuntimeError("sensitivity_matrix: the node matrix of scenarios %s is not "

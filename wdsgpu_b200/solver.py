@@ -299,6 +299,7 @@ class GGASolver:
         self.r_hw = torch.as_tensor(np.asarray(net.r_hw, dtype=np.float64), device=self.device)
         self._plans = []
         self._zeros = {}
+        self._off_pumps = None
 
     # ------------------------------------------------------------ set-up
     @staticmethod
@@ -625,10 +626,13 @@ class GGASolver:
             return 0.0
         return 1e-5
 
-    def pump_rows(self, B, speed=None, pump_h0=None, pump_r=None):
+    def pump_rows(self, B, speed=None, pump_h0=None, pump_r=None, later=None):
         """Pump parameters of a call as FP64 device rows: (speed, h0, r), each
         None or [1, L] / [B, L] with one common row count (an [L] row next to
-        [B, L] rows is expanded).  Values off pump links are not read."""
+        [B, L] rows is expanded).  Values off pump links are not read.  With a
+        list `later`, the comparison of speed with the link settings off pump
+        links is appended to it as a function to call once the host waits for
+        the call's results anyway."""
         vals = [speed, pump_h0, pump_r]
         if all(v is None for v in vals):
             return None
@@ -649,17 +653,32 @@ class GGASolver:
                 # the reference's speed is the whole link-setting vector
                 # (LinkSetting, dgga/autodiff.py:99-120); off pump links it
                 # would set valve settings, which this route does not take
-                off = self._lt != PUMP
-                host = t.cpu().numpy()
-                bad = np.flatnonzero((host[:, off] != self.init_setting[off]).any(0))
-                if bad.size:
-                    raise NotImplementedError(
-                        "speed differs from the network's link settings off pump links "
-                        "(links %s): valve settings are not parameters of this route"
-                        % np.flatnonzero(off)[bad][:8].tolist())
+                check = self._speed_check(t)
+                if later is None:
+                    check()
+                else:
+                    later.append(check)
             out.append(t)
         rows = max(t.shape[0] for t in out if t is not None)
         return tuple(None if t is None else t.expand(rows, L).contiguous() for t in out)
+
+    def _speed_check(self, t):
+        """Compares speed rows [., L] with the link settings off pump links, on
+        the device; the returned function reads the result and raises."""
+        if self._off_pumps is None:
+            self._off_pumps = (torch.as_tensor(self._lt != PUMP, device=self.device),
+                               torch.as_tensor(self.init_setting, device=self.device))
+        off, ref = self._off_pumps
+        hit = ((t != ref) & off).any()
+
+        def check():
+            if bool(hit):
+                bad = torch.nonzero(((t != ref) & off).any(0)).flatten()
+                raise NotImplementedError(
+                    "speed differs from the network's link settings off pump links "
+                    "(links %s): valve settings are not parameters of this route"
+                    % bad[:8].tolist())
+        return check
 
     def run(self, d, rh, ke, r, B, max_iter, hacc, status_machine, polish_steps,
             refine=None, plan=None, q0=None, e0=None, pumps=None, refine_band=None,
@@ -780,12 +799,13 @@ class GGASolver:
         o = self.run(d, rh, ke, r, B, max_iter, hacc, sm, -1, q0=q0, e0=e0,
                      schedule=bool(record_schedule))
         info = o["info"]
-        _check_info_flags(self, info)
-        bad = torch.nonzero(info & _lib.INFO_NOT_PD).flatten()
-        if bad.numel():
-            raise RuntimeError(
-                "batched LDL^T failed: the node matrix of scenarios %s is not "
-                "positive definite%s" % (bad.tolist(), _not_pd_hint(self)))
+        if info.cpu().numpy().any():   # the call's one host read: nothing to report when 0
+            _check_info_flags(self, info)
+            bad = torch.nonzero(info & _lib.INFO_NOT_PD).flatten()
+            if bad.numel():
+                raise RuntimeError(
+                    "batched LDL^T failed: the node matrix of scenarios %s is not "
+                    "positive definite%s" % (bad.tolist(), _not_pd_hint(self)))
         out = dict(head_ft=o["head"], flow_cfs=o["flow"], emitter_cfs=o["emit"],
                    iters=o["iters"].to(torch.int64), relerr=o["relerr"],
                    converged=(info == 0))
