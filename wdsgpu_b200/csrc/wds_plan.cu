@@ -145,7 +145,9 @@ struct WdsPlan {
   int rows_slots = 0;
   int max_batch = 0;
   int threads = 256;
-  int groups = 1;
+  int groups = 1;      // scenario groups per CTA at most
+  bool tuned = false;  // ... chosen by the caller: taken for every batch
+  int sms = 1;
   size_t smem_fwd = 0, smem_adj = 0;
   int nnzA_lower = 0;
   bool have_state = false;
@@ -155,6 +157,16 @@ struct WdsPlan {
   // tell whether its kept state is still the plan's
   int64_t gen = 0;
 };
+
+// Scenario groups per CTA of a launch of `batch` scenarios: as few as give
+// every scenario a place in the first round, up to the plan's count.  A CTA of
+// one group compiles to 255 registers per thread without spills, three groups
+// to 80 with spills, so a batch within the SM count runs faster in CTAs of one
+// group (542 junctions B=97: 289 -> 262 us of k_forward).
+static int groups_for(const WdsPlan* plan, int batch) {
+  if (plan->tuned) return plan->groups;
+  return std::min(plan->groups, std::max(1, (batch + plan->sms - 1) / plan->sms));
+}
 
 extern "C" const char* wds_last_error(void) { return g_err.c_str(); }
 
@@ -789,29 +801,27 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     d.msm = d.nT > 0 ? 1 : 0;
     d.sm_state = (int)std::min<size_t>(state_smem_bytes(d), 227 * 1024);
   } else {
-    // the top block's inverse goes to shared memory where that leaves as many
-    // scenarios resident (a substitution reads it once: 4 k cycles from L2,
-    // 1.5 k from shared memory, one group per SM, 36 columns), else to L2
-    auto resident = [&](int msm, int g) {  // scenarios per SM; 0: does not fit
+    // As many groups as fit (a CTA takes the SM's registers whatever its
+    // count, so one CTA per SM runs).  The top block's inverse goes to shared
+    // memory where that costs no group (a substitution reads it once: 4 k cycles
+    // from L2, 1.5 k from shared memory, one group per SM, 36 columns), else to L2.
+    auto fits = [&](int msm, int g) {
       d.msm = msm;
-      const size_t sm = (size_t)d.stab_bytes + g * state_smem_bytes(d);
-      if (sm > 227 * 1024) return 0;
-      return g * std::min((int)((228 * 1024) / (sm + 1024)), 2048 / (256 * g));
+      return (size_t)d.stab_bytes + g * state_smem_bytes(d) <= 227 * 1024;
     };
-    int best_g = 0, best_res = 0, msm = 0;
-    for (int g = 1; g <= 4; ++g)
-      for (int m = d.nT > 0 ? 1 : 0; m >= 0; --m)
-        if (resident(m, g) > best_res) { best_res = resident(m, g); best_g = g; msm = m; }
+    int best_g = 4;
+    while (best_g > 0 && !fits(0, best_g)) --best_g;
     if (net->groups_per_cta > 0) {  // a tuned choice, if the state fits
-      if (resident(0, net->groups_per_cta) == 0) {
+      if (!fits(0, net->groups_per_cta)) {
         cudaFree(plan->dtab);
         delete plan;
         return fail(WDS_E_ARG, "wds_plan: groups_per_cta " + std::to_string(net->groups_per_cta) +
                                    " exceeds shared memory for this network");
       }
       best_g = net->groups_per_cta;
-      msm = d.nT > 0 && resident(1, best_g) == resident(0, best_g) ? 1 : 0;
+      plan->tuned = true;
     }
+    const int msm = d.nT > 0 && best_g > 0 && fits(1, best_g) ? 1 : 0;
     d.msm = msm;
     const size_t st = state_smem_bytes(d);
     plan->groups = best_g;
@@ -823,6 +833,15 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     delete plan;
     return fail(WDS_E_UNSUPPORTED,
                 "wds_plan: the network's per-scenario state exceeds shared memory");
+  }
+  {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&plan->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+      cudaFree(plan->dtab);
+      delete plan;
+      return fail(WDS_E_CUDA, "wds_plan: device query failed");
+    }
   }
   // ---- workspace
   plan->max_batch = max_batch;
@@ -923,7 +942,7 @@ extern "C" int wds_forward(WdsPlan* plan, int32_t batch, const WdsForwardOpts* o
   a.head = head; a.flow = flow; a.emit = emitter; a.status = status; a.iters = iters;
   a.relerr = relerr; a.info = info;
   std::string err;
-  int rc = launch_forward(plan->dn, plan->dw, a, plan->groups, stream, &err);
+  int rc = launch_forward(plan->dn, plan->dw, a, groups_for(plan, batch), stream, &err);
   if (rc != WDS_OK) return fail(rc, err);
   plan->have_state = o->polish_steps >= 0;
   plan->state_batch = batch;
@@ -949,7 +968,7 @@ extern "C" int wds_adjoint_rhs(WdsPlan* plan, int32_t batch, int32_t rhs_per, in
   a.rhs_per = rhs_per;
   a.v0 = first;
   std::string err;
-  int rc = launch_adjoint(plan->dn, plan->dw, a, plan->groups, stream, &err);
+  int rc = launch_adjoint(plan->dn, plan->dw, a, groups_for(plan, batch), stream, &err);
   if (rc != WDS_OK) return fail(rc, err);
   return WDS_OK;
 }
@@ -978,10 +997,11 @@ extern "C" int wds_sensitivity(WdsPlan* plan, int32_t rows, int32_t rhs_per, int
   const size_t st = state_smem_bytes(d);
   const size_t scr = d.npcv > 0 ? ((size_t)w.nscr * d.Nj * 8 + 255) / 256 * 256 : 0;
   const size_t glob = d.wide && st > (size_t)d.sm_state ? (st + 255) / 256 * 256 : 0;
+  const int groups = groups_for(plan, rows);
   if (scr + glob > 0) {
-    const int grid = adjoint_grid(d, plan->groups, rows, &err);
+    const int grid = adjoint_grid(d, groups, rows, &err);
     if (grid < 0) return fail(WDS_E_CUDA, err);
-    const int slots = grid * plan->groups;
+    const int slots = grid * groups;
     if (slots > plan->rows_slots) {
       if (plan->drows) cudaFree(plan->drows);
       plan->drows = nullptr;
@@ -993,7 +1013,7 @@ extern "C" int wds_sensitivity(WdsPlan* plan, int32_t rows, int32_t rhs_per, int
     if (scr) w.scr = (double*)plan->drows;
     if (glob) w.state = (unsigned char*)plan->drows + (size_t)plan->rows_slots * scr;
   }
-  const int rc = launch_adjoint(d, w, a, plan->groups, stream, &err);
+  const int rc = launch_adjoint(d, w, a, groups, stream, &err);
   if (rc != WDS_OK) return fail(rc, err);
   return WDS_OK;
 }
@@ -1084,7 +1104,7 @@ extern "C" int wds_adjoint(WdsPlan* plan, int32_t batch, const double* gH, const
     return fail(WDS_E_STATE, "wds_adjoint: no implicit forward of this batch size to differentiate");
   AdjArgs a{batch, gH, gQ, gE, gd, grh, gke, gr};
   std::string err;
-  int rc = launch_adjoint(plan->dn, plan->dw, a, plan->groups, stream, &err);
+  int rc = launch_adjoint(plan->dn, plan->dw, a, groups_for(plan, batch), stream, &err);
   if (rc != WDS_OK) return fail(rc, err);
   return WDS_OK;
 }
@@ -1105,7 +1125,7 @@ extern "C" int wds_adjoint_pumps(WdsPlan* plan, int32_t batch, const double* gH,
   a.gh0 = gh0;
   a.grp = grp;
   std::string err;
-  int rc = launch_adjoint(plan->dn, plan->dw, a, plan->groups, stream, &err);
+  int rc = launch_adjoint(plan->dn, plan->dw, a, groups_for(plan, batch), stream, &err);
   if (rc != WDS_OK) return fail(rc, err);
   return WDS_OK;
 }
@@ -1133,7 +1153,7 @@ extern "C" int wds_unrolled_adjoint(WdsPlan* plan, int32_t batch, int32_t K,
   u.ke_stride = ke_stride; u.r = r; u.r_stride = r_stride; u.gH = gH; u.gQ = gQ; u.gE = gE;
   u.gd = gd; u.grh = grh; u.gke = gke; u.gr = gr; u.scr = scratch; u.s0 = status0;
   std::string err;
-  const int rc = launch_unrolled(plan->dn, plan->dw, u, plan->groups, stream, &err);
+  const int rc = launch_unrolled(plan->dn, plan->dw, u, groups_for(plan, batch), stream, &err);
   plan->have_state = false;  // the reverse pass reuses the plan's factor workspace
   ++plan->gen;
   if (rc != WDS_OK) return fail(rc, err);
@@ -1227,7 +1247,7 @@ extern "C" int wds_forward_noalloc(const WdsPlan* plan, int32_t batch, const Wds
   a.head = head; a.flow = flow; a.emit = emitter; a.status = status; a.iters = iters;
   a.relerr = relerr; a.info = info;
   std::string err;
-  rc = launch_forward(d, w, a, plan->groups, stream, &err);
+  rc = launch_forward(d, w, a, groups_for(plan, batch), stream, &err);
   if (rc != WDS_OK) return fail(rc, err);
   return WDS_OK;
 }
