@@ -56,7 +56,8 @@ constexpr double kReuseFlow = 1e-6;
 struct Sh {
   double *q, *P, *Y, *W, *V0, *V1, *V2, *hf, *xf, *red, *small;
   float* Wf;                      // the factor when it is kept in FP32 (W is then null)
-  double *em_e, *em_ke, *em_emh;  // per emitter slot: flow, coefficient, 1/hgrad
+  // per emitter slot: flow, coefficient, 1/hgrad, head loss, elevation
+  double *em_e, *em_ke, *em_emh, *em_hl, *em_el;
   int16_t* eslot;                 // [Nj] emitter slot of a junction or -1
   double* tb;                     // scratch of the top-block inversion (V2's storage)
   double* Mg;                     // [nT][top_ld(nT)] top-block inverse (shared memory when n.msm, else global)
@@ -234,7 +235,9 @@ __device__ void block_maxmin(double& mx, double& mn, double* red) {
 __device__ __forceinline__ void emitter_hl(const DevNet& n, double e, double ke, double& hl,
                                            double& hg) {
   const double kea = fmax(ke, kCSMALL);
-  hg = n.qexp * kea * pow(fmax(fabs(e), 1e-30), n.qexp - 1.0);
+  const double ea = fmax(fabs(e), 1e-30);
+  // (the default exponent 2 needs no power: pow(x, 1) = x)
+  hg = n.qexp * kea * (n.qexp == 2.0 ? ea : pow(ea, n.qexp - 1.0));
   const bool lin = hg < n.rqtol;
   if (lin) hg = n.rqtol;
   hl = lin ? hg * e : hg * e / n.qexp;
@@ -1050,101 +1053,90 @@ __device__ void dense_solve(double* C, double* y, int m) {
 }
 
 // ---------------------------------------------------------------- assembly
-// GGA assembly (linkcoeffs -> emittercoeffs -> nodecoeffs, solver.py:2958-3007)
-// into W (pattern of L) and F = V0; Xflow saved for PRV downstream nodes.
-template <int NT, class FT, class TB>
-__device__ void assemble_gga(const DevNet& n, const TB& T, const Sh& s, const double* kerow,
-                             const double* dj) {
+// Headloss stage of a GGA iteration (dgga/solver.py:2923-2956): P and Y of every
+// link, and 1/hgrad and head loss of every emitter.  What a link adds to the
+// right-hand side at its ends is formed here too, once, into the solves'
+// temporary: +Z at its first end and -Z at its second, Z = Y - q plus the
+// grounding term P H of a fixed end (a link with one fixed end reaches one
+// junction only); 0 for the control valves, which the valve pass adds.  The
+// node pass then reads P and Z from shared memory where it used to gather q
+// and Y from L2 and to test every incidence entry for valves and fixed ends (782
+// junctions, three groups per SM: 18.5 -> 4.7 k cycles an iteration).
+template <int NT, class TB>
+__device__ void link_pass(const DevNet& n, const PumpTh& th, const TB& T, const Sh& s,
+                          const double* rrow) {
   const int tid = gtid<NT>();
+  double* Z = s.V2;
+  // the next link's flow and resistance, in L2, are loaded while this link's
+  // coefficients are formed
+  int k = tid;
+  double qn = k < n.L ? s.q[k] : 0.0, rn = k < n.L ? rrow[k] : 0.0;
+  for (; k < n.L; k += NT) {
+    const double qk = qn, rk = rn;
+    const int kn = k + NT;
+    if (kn < n.L) {
+      qn = s.q[kn];
+      rn = rrow[kn];
+    }
+    double P, Y;
+    link_coef(n, th, k, qk, s.S[k], rk, false, P, Y);
+    s.P[k] = P;
+    s.Y[k] = Y;
+    const int c1 = T.e1[k], c2 = T.e2[k];
+    double z = Y - qk;
+    if (c2 < 0 && c1 >= 0) z += P * s.hf[-c2 - 1];
+    if (c1 < 0 && c2 >= 0) z -= P * s.hf[-c1 - 1];
+    const int kd = n.kind[k];
+    Z[k] = kd == WDS_KIND_PRV || kd == WDS_KIND_PSV || kd == WDS_KIND_FCV ? 0.0 : z;
+  }
+  for (int es = tid; es < s.flag[2]; es += NT) {
+    double hl, hg;
+    emitter_hl(n, s.em_e[es], s.em_ke[es], hl, hg);
+    s.em_hl[es] = hl;
+    s.em_emh[es] = 1.0 / hg;
+  }
+}
+
+// Assembly of the node matrix and right-hand side (linkcoeffs ->
+// emittercoeffs -> nodecoeffs, solver.py:2958-3007) from the link pass, into W
+// (pattern of L) and F = V0; Xflow saved for the junctions whose valves read it.
+template <int NT, class FT, class TB>
+__device__ void assemble_gga(const DevNet& n, const TB& T, const Sh& s, const double* dj) {
+  const int tid = gtid<NT>();
+  const double* Z = s.V2;
   for (int p = tid; p < n.Nj; p += NT) {
     const int a = T.inc_ptr[p], m = T.inc_split[p], z = T.inc_ptr[p + 1];
-    // the junction's global values are requested before its incidence sums
-    const double dem = dj[p];
-    const int xfs = n.node_xf[p];
-    double dg = 0.0, xf = 0.0, F = 0.0;
-    // the link flows and Y live in L2: the first kPre incident links' values
-    // are requested together, then summed in the reference's order (n1 side,
-    // then n2 side); a junction with more links loads the rest one by one
-    constexpr int kPre = 4;
-    double qv[kPre], yv[kPre];
-#pragma unroll
-    for (int u = 0; u < kPre; ++u) {
-      qv[u] = yv[u] = 0.0;
-      if (a + u < z) {
-        const int k = T.inc[a + u] & 0xffff;
-        qv[u] = s.q[k];
-        yv[u] = s.Y[k];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kPre; ++u) {
-      const int e = a + u;
-      if (e >= m) break;
-      const uint32_t ie = T.inc[e];
-      if (ie & (1u << 16)) continue;
-      dg += s.P[ie & 0xffff];
-      xf += -qv[u];
-      F += yv[u];
-    }
-    for (int e = a + kPre; e < m; ++e) {
-      const uint32_t ie = T.inc[e];
-      if (ie & (1u << 16)) continue;
-      const int k = ie & 0xffff;
+    const double dem = dj[p];  // (L2) requested before the incidence sums
+    const int es = s.eslot[p];
+    double dg = 0.0, F = 0.0;
+    for (int e = a; e < z; ++e) {
+      const int k = inc_link(T, e);
       dg += s.P[k];
-      xf += -s.q[k];
-      F += s.Y[k];
+      F += e < m ? Z[k] : -Z[k];
     }
-#pragma unroll
-    for (int u = 0; u < kPre; ++u) {
-      const int e = a + u;
-      if (e < m || e >= z) continue;
-      const uint32_t ie = T.inc[e];
-      if (ie & (1u << 16)) continue;
-      dg += s.P[ie & 0xffff];
-      xf += qv[u];
-      F += -yv[u];
+    if (es >= 0) {
+      const double emh = s.em_emh[es];
+      dg = dg + emh;
+      F = F + (s.em_hl[es] + s.em_el[es]) * emh - s.em_e[es];
     }
-    for (int e = (m > a + kPre ? m : a + kPre); e < z; ++e) {
+    wp<FT>(s)[T.colptr[p]] = (FT)dg;
+    s.V0[p] = F - dem;
+  }
+  for (int i = NT - 1 - tid; i < n.nxf; i += NT) {  // flow excess of the held junctions
+    const int p = n.xf_node[i], m = T.inc_split[p], z = T.inc_ptr[p + 1];
+    double xf = 0.0;
+    for (int e = T.inc_ptr[p]; e < z; ++e) {
       const uint32_t ie = T.inc[e];
-      if (ie & (1u << 16)) continue;
-      const int k = ie & 0xffff;
-      dg += s.P[k];
-      xf += s.q[k];
-      F += -s.Y[k];
-    }
-    for (int e = m; e < z; ++e) {  // n1 end fixed: F[Row[n2]] += P*H[n1]
-      const uint32_t ie = T.inc[e];
-      if ((ie & (1u << 16)) || !(ie & (1u << 17))) continue;
-      F += s.P[ie & 0xffff] * s.hf[ie >> 18];
-    }
-    for (int e = a; e < m; ++e) {  // n2 end fixed: F[Row[n1]] += P*H[n2]
-      const uint32_t ie = T.inc[e];
-      if ((ie & (1u << 16)) || !(ie & (1u << 17))) continue;
-      F += s.P[ie & 0xffff] * s.hf[ie >> 18];
+      const double q = ie & (1u << 16) ? 0.0 : s.q[ie & 0xffff];
+      xf += e < m ? -q : q;
     }
     const int es = s.eslot[p];
-    if (es >= 0) {
-      double hl, hg;
-      emitter_hl(n, s.em_e[es], s.em_ke[es], hl, hg);
-      const double emh = 1.0 / hg;
-      s.em_emh[es] = emh;
-      dg = dg + emh;
-      F = F + (hl + n.el[p]) / hg;
-      xf = xf - s.em_e[es];
-    }
-    xf = xf - dem;
-    F = F + xf;
-    wp<FT>(s)[T.colptr[p]] = (FT)dg;
-    s.V0[p] = F;
-    if (xfs >= 0) s.xf[xfs] = xf;
+    if (es >= 0) xf -= s.em_e[es];
+    s.xf[i] = xf - dj[p];
   }
   for (int t = tid; t < n.npairs; t += NT) {
     double v = 0.0;
-    for (int e = T.pptr[t]; e < T.pptr[t + 1]; ++e) {
-      const int pl = T.plink[e];
-      if (pl & 0x8000) continue;
-      v += -s.P[pl];
-    }
+    for (int e = T.pptr[t]; e < T.pptr[t + 1]; ++e) v += -s.P[T.plink[e] & 0x7fff];
     wp<FT>(s)[T.pslot[t]] = (FT)v;
   }
   for (int t = tid; t < n.nfill; t += NT) wp<FT>(s)[T.fill[t]] = FT(0);
@@ -1262,6 +1254,7 @@ __device__ void adj_coeffs(const DevNet& n, const PumpTh& th, const Sh& s, const
     double hl, hg;
     emitter_hl(n, s.em_e[es], s.em_ke[es], hl, hg);
     const double emh = 1.0 / hg;
+    s.em_hl[es] = hl;
     s.em_emh[es] = emh;
     if (Ef) fr = fr || !(fabs(emh - e0) <= tol * fabs(e0));
   }
@@ -1391,9 +1384,11 @@ __device__ void primal_solve(const DevNet& n, const TB& T, const Sh& s, double* 
   gsync<NT>();
 }
 
-// doubles of V2: a node vector, or the top-block inversion's scratch
+// doubles of V2: a node vector, a link vector (the link pass), or the top-block
+// inversion's scratch
 __host__ __device__ inline int v2_len(const DevNet& n) {
-  return n.nT > 0 && n.Nj < kTopScratch ? kTopScratch : n.Nj;
+  const int m = n.Nj > n.L ? n.Nj : n.L;
+  return n.nT > 0 && m < kTopScratch ? kTopScratch : m;
 }
 
 __host__ __device__ __forceinline__ size_t al16(size_t x) { return (x + 15) / 16 * 16; }
@@ -1418,6 +1413,8 @@ __host__ __device__ __forceinline__ Sh place_state(const DevNet& n, Take&& take)
   s.em_e = (double*)take(8ull * n.emcap);
   s.em_ke = (double*)take(8ull * n.emcap);
   s.em_emh = (double*)take(8ull * n.emcap);
+  s.em_hl = (double*)take(8ull * n.emcap);
+  s.em_el = (double*)take(8ull * n.emcap);
   // the solves' temporary; idle while the matrix is factored, so the top
   // block's inversion works there
   s.V2 = (double*)take(8ull * v2_len(n));
@@ -1503,6 +1500,7 @@ __device__ bool build_emitters(const DevNet& n, const Sh& s, const double* val, 
         s.em_ke[slot] = v;
         s.em_e[slot] = 1.0;
         s.em_emh[slot] = 0.0;
+        s.em_el[slot] = n.el[p];
       } else {
         s.eslot[p] = -1;
         if (em) over = true;
@@ -1600,7 +1598,7 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
   int nextcheck = n.checkfreq;
   int iters = maxtrials + 1, info = WDS_INFO_UNCONVERGED;
   double relerr = 0.0;
-  double dratio = 0.0;  // diag_ratio of the last iteration's assembled matrix
+  bool ran = false;
   const int rec_w = n.L + 2 * n.Nj;  // unrolled record: q [L], e [Nj], H [Nj] per iteration
   double* recb = a.rec ? a.rec + (size_t)b * maxtrials * rec_w : nullptr;
   for (int it = 1; it <= (em_ok ? maxtrials : 0); ++it) {
@@ -1610,36 +1608,11 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
       for (int p = gtid<NT>(); p < n.Nj; p += NT)
         r[n.L + p] = s.eslot[p] >= 0 ? s.em_e[s.eslot[p]] : 0.0;
     }
-    // ---- headloss coefficients (the next link's flow and resistance, in L2,
-    // are loaded while this link's coefficients are formed)
-    {
-      int k = gtid<NT>();
-      double qn = k < n.L ? s.q[k] : 0.0, rn = k < n.L ? rrow[k] : 0.0;
-      for (; k < n.L; k += NT) {
-        const double qk = qn, rk = rn;
-        const int kn = k + NT;
-        if (kn < n.L) {
-          qn = s.q[kn];
-          rn = rrow[kn];
-        }
-        double P, Y;
-        link_coef(n, th, k, qk, s.S[k], rk, false, P, Y);
-        s.P[k] = P;
-        s.Y[k] = Y;
-      }
-    }
+    // ---- headloss coefficients, assembly
+    link_pass<NT>(n, th, T, s, rrow);
     gsync<NT>();
-    assemble_gga<NT, FT>(n, T, s, kerow, dj);
-    if (a.diag && n.npcv > 0) {  // condition proxy (dgga/solver.py:3026-3032)
-      double mx = 0.0, mn = kINF;
-      for (int p = gtid<NT>(); p < n.Nj; p += NT) {
-        const double dv = fabs((double)wp<FT>(s)[T.colptr[p]]);
-        mx = fmax(mx, dv);
-        mn = fmin(mn, dv);
-      }
-      block_maxmin<NT>(mx, mn, s.red);
-      dratio = mx / fmax(mn, 1e-300);
-    }
+    assemble_gga<NT, FT>(n, T, s, dj);
+    ran = true;
     if (!factor<NT, FT>(n, T, s)) {
       info = WDS_INFO_NOT_PD;
       iters = it;
@@ -1677,9 +1650,7 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
     for (int p = gtid<NT>(); p < n.Nj; p += NT) {
       const int es = s.eslot[p];
       if (es >= 0) {
-        double hl, hg;
-        emitter_hl(n, s.em_e[es], s.em_ke[es], hl, hg);
-        const double dqe = (hl - (s.V1[p] - n.el[p])) / hg;
+        const double dqe = (s.em_hl[es] - (s.V1[p] - s.em_el[es])) * s.em_emh[es];
         const double en = s.em_e[es] - dqe;
         s.em_e[es] = en;
         sums[2] += fabs(dqe);
@@ -1813,6 +1784,39 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
     info = 0;
   }
   gsync<NT>();
+  // condition proxy (dgga/solver.py:3026-3032) of the last iteration's matrix:
+  // its diagonal again from the last iteration's coefficients (P, 1/hgrad),
+  // into V0, in the order of the assembly
+  double dratio = 0.0;
+  if (a.diag && n.npcv > 0 && ran) {
+    double mx = 0.0, mn = kINF;
+    for (int p = gtid<NT>(); p < n.Nj; p += NT) {
+      double dg = 0.0;
+      for (int e = T.inc_ptr[p]; e < T.inc_ptr[p + 1]; ++e) {
+        const uint32_t ie = T.inc[e];
+        dg += ie & (1u << 16) ? 0.0 : s.P[ie & 0xffff];
+      }
+      if (s.eslot[p] >= 0) dg = dg + s.em_emh[s.eslot[p]];
+      s.V0[p] = dg;
+    }
+    gsync<NT>();
+    if (gtid<NT>() == 0)
+      for (int v = 0; v < n.npcv + n.nfcv; ++v) {
+        const int o = n.vord[v], f = -1 - o;
+        const int k = o < 0 ? n.fcv_link[f] : n.pcv_link[o];
+        s.V0[o < 0 ? n.fcv_j1[f] : n.pcv_j1[o]] += s.P[k];
+        s.V0[o < 0 ? n.fcv_j2[f] : n.pcv_j2[o]] += s.P[k];
+        if (o >= 0 && s.P[k] == 0.0) s.V0[n.pcv_jc[o]] += kCBIG;
+      }
+    gsync<NT>();
+    for (int p = gtid<NT>(); p < n.Nj; p += NT) {
+      const double dv = fabs(s.V0[p]);
+      mx = fmax(mx, dv);
+      mn = fmin(mn, dv);
+    }
+    block_maxmin<NT>(mx, mn, s.red);
+    dratio = mx / fmax(mn, 1e-300);
+  }
   // junction heads of the GGA solution stay in V1
   double* Hs = w.scr + (size_t)b * w.nscr * n.Nj;  // global copy of heads for the polish
   if (a.polish >= 0 && info == 0) {
@@ -1886,9 +1890,7 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
         const int es = s.eslot[p];
         double re = 0.0, emh = 0.0;
         if (es >= 0) {
-          double hl, hg;
-          emitter_hl(n, s.em_e[es], s.em_ke[es], hl, hg);
-          re = hl - (Hs[p] - n.el[p]);
+          re = s.em_hl[es] - (Hs[p] - s.em_el[es]);
           mm = mm - s.em_e[es];
           emh = s.em_emh[es];
         }
@@ -1916,10 +1918,8 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
       for (int p = gtid<NT>(); p < n.Nj; p += NT) {
         const int es = s.eslot[p];
         if (es >= 0) {
-          double hl, hg;
-          emitter_hl(n, s.em_e[es], s.em_ke[es], hl, hg);
-          const double re = hl - (Hs[p] - n.el[p]);
-          s.em_e[es] = s.em_e[es] + (-re + s.V1[p]) / hg;
+          const double re = s.em_hl[es] - (Hs[p] - s.em_el[es]);
+          s.em_e[es] = s.em_e[es] + (s.V1[p] - re) * s.em_emh[es];
         }
         Hs[p] = Hs[p] + s.V1[p];
       }
@@ -2393,14 +2393,9 @@ __device__ __forceinline__ void unrolled_one(const DevNet& n, const DevWork& w, 
       s.V1[p] = rr[n.L + n.Nj + p];
     }
     gsync<NT>();
-    for (int k = tid; k < n.L; k += NT) {
-      double P, Y;
-      link_coef(n, th, k, s.q[k], s.S[k], rrow[k], false, P, Y);
-      s.P[k] = P;
-      s.Y[k] = Y;
-    }
+    link_pass<NT>(n, th, T, s, rrow);
     gsync<NT>();
-    assemble_gga<NT, FT>(n, T, s, kerow, dj);
+    assemble_gga<NT, FT>(n, T, s, dj);
     factor<NT, FT>(n, T, s);  // the forward factored this matrix: positive definite
     // (1) q' = q - dq: the head-difference adjoint of each link
     for (int k = tid; k < n.L; k += NT) {

@@ -58,7 +58,7 @@ struct DevNet {
   const int* inc_ptr;     // [Nj+1]
   const int* inc_split;   // [Nj] first n2-side entry
   const int* inc;         // link index of each incidence entry
-  const int* node_xf;     // [Nj] Xflow save slot or -1
+  const int* xf_node;     // [nxf] junction of each Xflow slot
   const int* cb_ptr;      // [Nj+1] pcv valves whose downstream node is p
   const int* cb_idx;
   // fixed nodes [Nf]

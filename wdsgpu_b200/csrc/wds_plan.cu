@@ -441,7 +441,7 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
       if (!is_a[e]) fill_slot.push_back(e);
   // ---- status-machine PRVs
   // (PRVs and PSVs with a setting, in link order)
-  std::vector<int> link_pcv(L, -1), pcv_link, pcv_j1, pcv_j2, pcv_off, pcv_xf, node_xf(Nj, -1);
+  std::vector<int> link_pcv(L, -1), pcv_link, pcv_j1, pcv_j2, pcv_off, pcv_xf, node_xf(Nj, -1), xf_node;
   std::vector<int> pcv_jc, pcv_jo, pcv_psv;
   std::vector<double> pcv_hset, pcv_km, pcv_sgn;
   int nxf = 0;
@@ -461,7 +461,10 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     pcv_sgn.push_back(psv ? -1.0 : 1.0);
     pcv_psv.push_back(psv ? 1 : 0);
     pcv_off.push_back(pair_slot_of[{std::max(e1[k], e2[k]), std::min(e1[k], e2[k])}]);
-    if (node_xf[jc] < 0) node_xf[jc] = nxf++;
+    if (node_xf[jc] < 0) {
+      node_xf[jc] = nxf++;
+      xf_node.push_back(jc);
+    }
     pcv_xf.push_back(node_xf[jc]);
     pcv_hset.push_back(net->prv_hset[k]);
     pcv_km.push_back(net->km[k]);
@@ -578,7 +581,8 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
            in(fcv_link[f], 0, L);
     ok = ok && (int)vord.size() == npcv + nfcv;
     for (int v : vord) ok = ok && (v >= 0 ? v < npcv : (-1 - v) < nfcv);
-    for (int p = 0; p < Nj; ++p) ok = ok && node_xf[p] < std::max(nxf, 1);
+    ok = ok && (int)xf_node.size() == nxf;
+    for (int v : xf_node) ok = ok && in(v, 0, Nj);
     for (int t = 0; t < ntl; ++t) ok = ok && in(tl_tank[t], 0, Nf) && endok(tl_other[t]);
     for (int k = 0; k < L; ++k) {
       if (net->pump_type[k] == 2 && net->link_kind[k] == WDS_KIND_PUMP)
@@ -711,7 +715,7 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
          o_cptr = blob.add(cptr), o_cx = blob.add(cx), o_cy = blob.add(cy),
          o_ltl = blob.add(link_tl), o_lpcv = blob.add(link_pcv), o_jn = blob.add(jn),
          o_el = blob.add(el), o_incp = blob.add(inc_ptr), o_incs = blob.add(inc_split),
-         o_inc = blob.add(inc), o_nxf = blob.add(node_xf), o_cbp = blob.add(cb_ptr),
+         o_inc = blob.add(inc), o_nxf = blob.add(xf_node), o_cbp = blob.add(cb_ptr),
          o_cbi = blob.add(cb_idx), o_fn = blob.add(fnodes), o_fincp = blob.add(finc_ptr),
          o_fincs = blob.add(finc_split), o_finc = blob.add(finc), o_pp = blob.add(pair_ptr),
          o_pl = blob.add(pair_link), o_ps = blob.add(pair_slot), o_fs = blob.add(fill_slot),
@@ -762,7 +766,7 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
   d.cx = P_(double, o_cx); d.cy = P_(double, o_cy); d.link_tl = P_(int, o_ltl);
   d.link_pcv = P_(int, o_lpcv); d.jnode = P_(int, o_jn); d.el = P_(double, o_el);
   d.inc_ptr = P_(int, o_incp); d.inc_split = P_(int, o_incs); d.inc = P_(int, o_inc);
-  d.node_xf = P_(int, o_nxf); d.cb_ptr = P_(int, o_cbp); d.cb_idx = P_(int, o_cbi);
+  d.xf_node = P_(int, o_nxf); d.cb_ptr = P_(int, o_cbp); d.cb_idx = P_(int, o_cbi);
   d.fnode = P_(int, o_fn); d.finc_ptr = P_(int, o_fincp); d.finc_split = P_(int, o_fincs);
   d.finc = P_(int, o_finc); d.pair_ptr = P_(int, o_pp); d.pair_link = P_(int, o_pl);
   d.pair_slot = P_(int, o_ps); d.fill_slot = P_(int, o_fs); d.colptr = P_(int, o_cp);
