@@ -92,6 +92,16 @@ struct TabT {
   const uint16_t* plink;      // link | PRV << 15
   const Slot* pslot;          // [npairs]
   const Slot* fill;           // [nfill]
+  // large networks (kWide): factor entries, their terms, column records of the
+  // two substitutions, and the rounds of the factor and the substitutions (see factor_rounds)
+  const uint4* act;
+  const uint4* term;
+  const uint4* colf;
+  const uint4* colb;
+  const uint2* frnd;
+  const uint2* crnd;
+  const uint2* brnd;
+  const int* rptr3;           // [3][warps + 1] each warp's part of frnd, crnd, brnd
   const Slot* dslot;          // [nT (nT+1) / 2] slot of top-block entry (i >= j) or all ones
 
   // update list of the entry in `slot`: first term, term count, diagonal flag
@@ -150,6 +160,16 @@ __device__ TB tab_view(const DevNet& n, const unsigned char* b) {
   t.pslot = (const S*)(b + n.o_pslot);
   t.fill = (const S*)(b + n.o_fill);
   t.dslot = (const S*)(b + n.o_dslot);
+  if constexpr (TB::kWide) {
+    t.act = (const uint4*)(b + n.o_act);
+    t.term = (const uint4*)(b + n.o_term);
+    t.colf = (const uint4*)(b + n.o_colf);
+    t.colb = (const uint4*)(b + n.o_colb);
+    t.frnd = (const uint2*)(b + n.o_frnd);
+    t.crnd = (const uint2*)(b + n.o_crnd);
+    t.brnd = (const uint2*)(b + n.o_brnd);
+    t.rptr3 = (const int*)(b + n.o_rptr3);
+  }
   return t;
 }
 
@@ -527,6 +547,21 @@ __device__ __forceinline__ FT group_sum(FT v, int lg) {
   return v;
 }
 
+// 1 / x for a positive normal x to about one unit in the last place: the
+// hardware's 23-bit approximation and two Newton steps (48 cycles of latency
+// against 77 of the correctly rounded __drcp_rn, measured on dependent
+// chains).
+__device__ __forceinline__ double recip(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+
+// 1 / D of a pivot
+__device__ __forceinline__ double inv_pivot(double w) { return recip(w); }
+__device__ __forceinline__ float inv_pivot(float w) { return 1.0f / w; }
+
 // The factor of the scenario in its storage precision FT (double, or float
 // for the FP32 factor with FP64 refinement).
 template <class FT>
@@ -544,8 +579,8 @@ template <class TB, class FT>
 __device__ __forceinline__ void fac_range(const TB& T, FT* W, int t0, int t1, int lg, int t,
                                           int nthr, bool& bad) {
   const int G = 1 << lg, li = t & (G - 1), per = nthr >> lg;
-  for (int base = t0; base < t1; base += per) {
-    const int slot = base + (t >> lg);
+  for (int base = t0 + ((t & ~31) >> lg); base < t1; base += per) {  // a warp without items skips
+    const int slot = base + ((t & 31) >> lg);
     const bool valid = slot < t1;
     bool diag = false;
     FT acc = 0;
@@ -555,7 +590,7 @@ __device__ __forceinline__ void fac_range(const TB& T, FT* W, int t0, int t1, in
       const int pe = pb + cnt;
       for (int pr = pb + li; pr < pe; pr += G) {
         const auto* f = T.fpair + 3 * pr;
-        acc += W[f[0]] * W[f[1]] * W[f[2]];
+        acc = fma(W[f[0]] * W[f[1]], W[f[2]], acc);
       }
     }
     acc = group_sum(acc, lg);
@@ -563,7 +598,7 @@ __device__ __forceinline__ void fac_range(const TB& T, FT* W, int t0, int t1, in
       const FT w = W[slot] - acc;
       if (diag) {
         if (!(w > FT(0)) || !isfinite(w)) bad = true;
-        W[slot] = FT(1) / w;
+        W[slot] = inv_pivot(w);
       } else {
         W[slot] = w;
       }
@@ -577,8 +612,8 @@ template <class TB, class FT>
 __device__ __forceinline__ void fwd_range(const TB& T, const FT* W, double* v, int c0,
                                           int c1, int lg, int t, int nthr, bool top) {
   const int G = 1 << lg, li = t & (G - 1), per = nthr >> lg;
-  for (int base = c0; base < c1; base += per) {
-    const int j = base + (t >> lg);
+  for (int base = c0 + ((t & ~31) >> lg); base < c1; base += per) {
+    const int j = base + ((t & 31) >> lg);
     const bool valid = j < c1;
     FT acc = 0;
     if (valid) {
@@ -586,7 +621,7 @@ __device__ __forceinline__ void fwd_range(const TB& T, const FT* W, double* v, i
       for (int e = (int)T.rptr[j] + li; e < e1; e += G) {
         int sl, k;
         T.re(e, sl, k);
-        acc += W[sl] * (FT)v[k];
+        acc = fma(W[sl], (FT)v[k], acc);
       }
     }
     acc = group_sum(acc, lg);
@@ -603,18 +638,18 @@ template <class TB, class FT>
 __device__ __forceinline__ void bwd_level(const TB& T, const FT* W, double* v, int c0, int c1,
                                           int lg, int t, int nthr) {
   const int G = 1 << lg, li = t & (G - 1), per = nthr >> lg;
-  for (int base = c0; base < c1; base += per) {
-    const int j = base + (t >> lg);
+  for (int base = c0 + ((t & ~31) >> lg); base < c1; base += per) {
+    const int j = base + ((t & 31) >> lg);
     const bool valid = j < c1;
     int cb = 0;
     FT acc = 0;
     if (valid) {
       cb = T.colptr[j];
       const int ce = T.colptr[j + 1];
-      for (int e = cb + 1 + li; e < ce; e += G) acc += W[e] * (FT)v[T.rowidx[e]];
+      for (int e = cb + 1 + li; e < ce; e += G) acc = fma(W[e], (FT)v[T.rowidx[e]], acc);
     }
     acc = group_sum(acc, lg);
-    if (valid && li == 0) v[j] = (double)((FT)v[j] - W[cb] * acc);
+    if (valid && li == 0) v[j] = (double)fma(-W[cb], acc, (FT)v[j]);
   }
 }
 
@@ -658,17 +693,6 @@ __device__ __forceinline__ void top_wait(int id, int warps) {
                : "memory");
 }
 constexpr int kTopA = 5, kTopB = 9;
-
-// 1 / x for a positive normal x to about one unit in the last place: the
-// hardware's 23-bit approximation and two Newton steps (48 cycles of latency
-// against 77 of the correctly rounded __drcp_rn, measured on dependent
-// chains).
-__device__ __forceinline__ double recip(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = fma(y, fma(-x, y, 1.0), y);
-  return fma(y, fma(-x, y, 1.0), y);
-}
 
 // Inverse of the 4 x 4 pivot block at q (row-major), every lane the same (so
 // that nothing is broadcast); lane 0 writes it to pin.  The pivots come in pairs with one reciprocal each:
@@ -893,8 +917,20 @@ __device__ __noinline__ void top_apply(const double* Mg, double* vT, int nT) {
 // the columns below the top block; the top block's slots hold its Schur
 // complement and its inverse goes to s.Mg.  Returns true when every pivot was
 // positive and finite.
+template <int NT, class FT>
+__device__ bool factor_rounds(const uint2* rec, const int* ptr, const uint4* ent,
+                              const uint4* term, FT* W);
+template <int NT, bool BACK, class FT>
+__device__ void solve_rounds(const uint2* rec, const int* ptr, const uint4* cols, const uint2* rent,
+                             const uint16_t* rowidx, const FT* W, double* v);
+
 template <int NT, class FT, class TB>
 __device__ bool factor(const DevNet& n, const TB& T, const Sh& s) {
+  if constexpr (TB::kWide) {
+    bool bad = factor_rounds<NT, FT>(T.frnd, T.rptr3, T.act, T.term, wp<FT>(s));
+    if (n.nT > 0 && top_inverse<NT>((const FT*)wp<FT>(s), T.dslot, s.tb, s.Mg, n.nT)) bad = true;
+    return !gsync_or<NT>(bad);
+  } else {
   const int tid = gtid<NT>(), lane = tid & 31;
   const bool inw = in_narrow_warp<NT>();
   bool bad = false, prev_wide = true;
@@ -931,12 +967,20 @@ __device__ bool factor(const DevNet& n, const TB& T, const Sh& s) {
     if (top_inverse<NT>((const FT*)wp<FT>(s), T.dslot, s.tb, s.Mg, n.nT)) bad = true;
   }
   return !gsync_or<NT>(bad);
+  }
 }
 
 // In-place (L D L^T) v = b: forward levels below the top block, the top rows'
 // right-hand side, the dense top solve, backward levels below the top block.
 template <int NT, class FT, class TB>
 __device__ void solve(const DevNet& n, const TB& T, const Sh& s, double* v) {
+  if constexpr (TB::kWide) {
+    const uint2* re = reinterpret_cast<const uint2*>(T.rent);
+    solve_rounds<NT, false, FT>(T.crnd, T.rptr3 + NT / 32 + 1, T.colf, re, T.rowidx, wp<FT>(s), v);
+    if (n.nT > 0) top_apply<NT>(s.Mg, v + n.cT, n.nT);
+    solve_rounds<NT, true, FT>(T.brnd, T.rptr3 + 2 * (NT / 32 + 1), T.colb, re, T.rowidx, wp<FT>(s), v);
+    return;
+  } else {
   const int tid = gtid<NT>(), lane = tid & 31;
   const bool inw = in_narrow_warp<NT>();
   bool prev_wide = true;
@@ -991,6 +1035,170 @@ __device__ void solve(const DevNet& n, const TB& T, const Sh& s, double* v) {
     b1 = b0;
   }
   gsync<NT>();
+  }
+}
+
+// ---------------------------------------------------------------- large networks
+// The levels of a large network read their tables from L2, and 32 warps walk
+// every level, most of them without an item in the narrow upper ones.  Here a
+// pass is one list of rounds per warp, holding only the rounds in which the
+// warp has items (at most 32 >> lg), {first item, count | lg << 6 | top << 9 |
+// barriers << 16}: the warp passes the group barriers that lie between its
+// rounds (one between two levels unless one warp does both) and nothing else.
+// The tables are read ahead: the record three rounds, the item's record two
+// rounds, its first two terms per lane one round.  An item's sum is formed on
+// 1 << lg lanes as in the routines above.
+// Bound by issue and the L2 latency of lists longer than two entries a lane:
+// solve and gradient of 33 scenarios of 3000 junctions 3.08 -> 2.43 ms, 64
+// scenarios x 12 steps of 20 000 junctions 137 -> 111 ms (level loops over all
+// warps before; with the level's lane groups instead of the round's 2.82 and
+// 130 ms).
+
+// Item of this lane in round r, or -1.
+__device__ __forceinline__ int round_item(uint2 r) {
+  const int i = (int)(threadIdx.x & 31) >> ((r.y >> 6) & 7);
+  return i < (int)(r.y & 63u) ? (int)r.x + i : -1;
+}
+
+// The barriers before round r; rounds of one warp in a row need its own only.
+template <int NT>
+__device__ __forceinline__ void round_begin(uint2 r) {
+  __syncwarp();
+  for (int k = (int)(r.y >> 16); k > 0; --k) gsync<NT>();
+}
+
+// The LDL^T of the levels and the top block's Schur complement: ent holds
+// {first term, count | diagonal << 31, slot, 0}, term {L_ik, L_jk, 1/D_k, 0}
+// slots.  Returns whether a pivot was not positive and finite.
+template <int NT, class FT>
+__device__ __noinline__ bool factor_rounds(const uint2* rec, const int* ptr, const uint4* ent,
+                                           const uint4* term, FT* W) {
+  const uint2 none = make_uint2(0, 0);
+  const uint4 nil = make_uint4(0, 0, 0, 0);
+  const int w = gtid<NT>() >> 5, lane = threadIdx.x & 31, nr = ptr[w + 1] - ptr[w] - 1;
+  rec += ptr[w];  // the list ends with the barriers after the last round
+  bool bad = false;
+  auto entry = [&](uint2 r) {
+    const int i = round_item(r);
+    return i >= 0 ? ent[i] : nil;
+  };
+  auto terms = [&](uint4 s, uint2 r, uint4& a, uint4& b) {
+    const int l = (int)(r.y >> 6) & 7, li = lane & ((1 << l) - 1);
+    const int cnt = (int)(s.y & 0x7fffffffu);
+    a = li < cnt ? term[s.x + li] : nil;
+    b = li + (1 << l) < cnt ? term[s.x + li + (1 << l)] : nil;
+  };
+  uint2 r0 = rec[0], r1 = nr > 0 ? rec[1] : none, r2 = nr > 1 ? rec[2] : none;
+  uint4 s0 = entry(r0), s1 = entry(r1), a0, b0;
+  terms(s0, r0, a0, b0);
+  for (int i = 0; i < nr; ++i) {
+    const uint2 r3 = i + 3 <= nr ? rec[i + 3] : none;
+    const uint4 s2 = entry(r2);
+    uint4 a1, b1;
+    terms(s1, r1, a1, b1);
+    round_begin<NT>(r0);
+    const int lg = (int)(r0.y >> 6) & 7, G = 1 << lg, li = lane & (G - 1);
+    const int cnt = (int)(s0.y & 0x7fffffffu);
+    FT acc = 0;
+    if (li < cnt) acc = fma(W[a0.x] * W[a0.y], W[a0.z], acc);
+    if (li + G < cnt) acc = fma(W[b0.x] * W[b0.y], W[b0.z], acc);
+    for (int e = li + 2 * G; e < cnt; e += G) {
+      const uint4 f = term[s0.x + e];
+      acc = fma(W[f.x] * W[f.y], W[f.z], acc);
+    }
+    acc = group_sum(acc, lg);
+    if (round_item(r0) >= 0 && li == 0) {
+      const FT x = W[s0.z] - acc;
+      const bool diag = (s0.y >> 31) != 0;
+      if (diag && (!(x > FT(0)) || !isfinite(x))) bad = true;
+      W[s0.z] = diag ? inv_pivot(x) : x;
+    }
+    r0 = r1;
+    r1 = r2;
+    r2 = r3;
+    s0 = s1;
+    s1 = s2;
+    a0 = a1;
+    b0 = b1;
+  }
+  round_begin<NT>(r0);
+  return bad;
+}
+
+// Forward substitution (BACK false: entries {slot, column} of the column's row)
+// or backward substitution (BACK true: the column's own entries, rows in
+// rowidx) in v; column records {first row entry, entries, diagonal slot, column}.
+template <int NT, bool BACK, class FT>
+__device__ __noinline__ void solve_rounds(const uint2* rec, const int* ptr, const uint4* cols,
+                                          const uint2* rent, const uint16_t* rowidx,
+                                          const FT* W, double* v) {
+  const uint2 none = make_uint2(0, 0);
+  const uint4 nil = make_uint4(0, 0, 0, 0);
+  const int w = gtid<NT>() >> 5, lane = threadIdx.x & 31, nr = ptr[w + 1] - ptr[w] - 1;
+  rec += ptr[w];
+  auto column = [&](uint2 r) {
+    const int j = round_item(r);
+    return j >= 0 ? cols[j] : nil;
+  };
+  // entry e of the column: its slot and the index of its vector element
+  auto entry = [&](uint4 c, int e, int& sl, int& k) {
+    if constexpr (BACK) {
+      sl = (int)c.z + 1 + e;
+      k = rowidx[sl];
+    } else {
+      const uint2 x = rent[c.x + e];
+      sl = (int)x.x;
+      k = (int)x.y;
+    }
+  };
+  auto first2 = [&](uint4 c, uint2 r, int& sa, int& ka, int& sb, int& kb) {
+    const int l = (int)(r.y >> 6) & 7, li = lane & ((1 << l) - 1), n = (int)c.y;
+    sa = ka = sb = kb = 0;
+    if (li < n) entry(c, li, sa, ka);
+    if (li + (1 << l) < n) entry(c, li + (1 << l), sb, kb);
+  };
+  uint2 r0 = rec[0], r1 = nr > 0 ? rec[1] : none, r2 = nr > 1 ? rec[2] : none;
+  uint4 c0 = column(r0), c1 = column(r1);
+  int sa, ka, sb, kb;
+  first2(c0, r0, sa, ka, sb, kb);
+  FT wa = W[sa], wb = W[sb], wd = W[c0.z];
+  for (int i = 0; i < nr; ++i) {
+    const uint2 r3 = i + 3 <= nr ? rec[i + 3] : none;
+    const uint4 c2 = column(r2);
+    int sa1, ka1, sb1, kb1;
+    first2(c1, r1, sa1, ka1, sb1, kb1);
+    round_begin<NT>(r0);
+    const int lg = (int)(r0.y >> 6) & 7, G = 1 << lg, li = lane & (G - 1), n = (int)c0.y;
+    FT acc = 0;
+    if (li < n) acc = fma(wa, (FT)v[ka], acc);
+    if (li + G < n) acc = fma(wb, (FT)v[kb], acc);
+    for (int e = li + 2 * G; e < n; e += G) {
+      int sl, k;
+      entry(c0, e, sl, k);
+      acc = fma(W[sl], (FT)v[k], acc);
+    }
+    acc = group_sum(acc, lg);
+    if (round_item(r0) >= 0 && li == 0) {
+      const int j = (int)c0.w;
+      if constexpr (BACK) {
+        v[j] = (double)fma(-wd, acc, (FT)v[j]);
+      } else {
+        const FT x = (FT)v[j] - acc;
+        v[j] = (double)((r0.y >> 9) & 1u ? x : x * wd);
+      }
+    }
+    wa = W[sa1];
+    wb = W[sb1];
+    wd = W[c1.z];
+    ka = ka1;
+    kb = kb1;
+    r0 = r1;
+    r1 = r2;
+    r2 = r3;
+    c0 = c1;
+    c1 = c2;
+  }
+  round_begin<NT>(r0);
 }
 
 // x = A^{-1} rhs with `refine` refinement steps against the matrix-free A.

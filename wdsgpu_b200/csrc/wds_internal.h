@@ -124,6 +124,8 @@ struct DevNet {
   const uint4* stab;
   int stab_bytes;
   int o_spair, o_fpair, o_colptr, o_rowidx, o_levptr, o_rptr, o_rent, o_mode, o_inc_ptr, o_inc_split, o_inc, o_e1, o_e2, o_pptr, o_plink, o_pslot, o_fill, o_dslot;
+  // large networks: see factor_rounds
+  int o_act, o_term, o_colf, o_colb, o_frnd, o_crnd, o_brnd, o_rptr3;
   // dense top block: levels [L0, nlev) = columns [cT, Nj), nT = Nj - cT
   // (nT = 0 and L0 = nlev when the network has none)
   int L0, cT, nT;

@@ -638,7 +638,124 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
                                           net->link_kind[pair_link[e]] == WDS_KIND_FCV ||
                                           net->link_kind[pair_link[e]] == WDS_KIND_PSV) ? 0x8000 : 0));
   if (s_pl.empty()) s_pl.push_back(0);
-  struct TabOff { int sp, fp, cp, ri, lp, rp, re, md, ip, is, in, e1, e2, pp, pl, ps, fl, ds; };
+  // ---- large networks: the levels as rounds (see factor_rounds).  Factor
+  // entries: the diagonals below the top block and the entries with updates.
+  std::vector<uint4> wact, wterm, wcf, wcb;
+  std::vector<uint2> wfr, wcr, wbr;
+  std::vector<int> wptr;
+  // `same`: the network has the small layout too, and sums its items on the
+  // lanes that layout gives them (the layouts then agree bitwise); otherwise the
+  // items of a level are sorted by their lists' lengths and each round takes
+  // the lanes that suit it.
+  auto large_tables = [&](bool same) {
+    constexpr int nw = kWideThreads / 32;
+    struct Round { int a, n, lg; };
+    struct LevelRounds { std::vector<Round> r; bool narrow, top; };
+    std::vector<LevelRounds> lv;
+    // Rounds of items with the lists `len` (descending unless `same`), first
+    // item a: lanes enough that a list is at most k entries a lane, k by the
+    // level's instructions on four schedulers and its slowest round (about 350
+    // cycles per entry beyond the two read ahead).
+    auto add_level = [&](int a, const std::vector<int>& len, uint8_t md, bool top) {
+      LevelRounds best{{}, false, top};
+      const int n = (int)len.size();
+      if (same) {
+        best.narrow = !(md & 0x80);
+        const int lg = md & 7;
+        for (int i = 0; i < n; i += 32 >> lg) best.r.push_back({a + i, std::min(n - i, 32 >> lg), lg});
+      } else {
+        double cost = 1e300;
+        for (const int k : {2, 3, 4, 6, 8, 12, 16, 1 << 20}) {
+          std::vector<Round> r;
+          double all = 0.0, slow = 0.0;
+          for (int i = 0; i < n;) {
+            int lg = 0;
+            while (lg < 5 && (len[i] + (1 << lg) - 1) >> lg > k) ++lg;
+            const int per = (len[i] + (1 << lg) - 1) >> lg, c = std::min(n - i, 32 >> lg);
+            r.push_back({a + i, c, lg});
+            all += 60.0 + 9.0 * lg + 14.0 * per;
+            slow = std::max(slow, 6.0 * (60.0 + 9.0 * lg) + 350.0 * std::max(per - 2, 0));
+            i += c;
+          }
+          if (all / 4.0 + slow < cost) { cost = all / 4.0 + slow; best.r = r; }
+        }
+        best.narrow = best.r.size() <= 1;
+      }
+      lv.push_back(best);
+    };
+    // the warps' lists of a pass over the levels lv
+    auto rounds = [&](std::vector<uint2>& out) {
+      std::vector<std::vector<uint2>> per(nw);
+      std::vector<int> seen(nw, 0);  // barriers before the warp's next round
+      int bars = 0;
+      for (size_t l = 0; l < lv.size(); ++l) {
+        if (l > 0 && !(lv[l].narrow && lv[l - 1].narrow)) ++bars;
+        int w = 0;
+        for (const Round& r : lv[l].r) {
+          per[w].push_back(make_uint2((uint32_t)r.a, (uint32_t)r.n | (uint32_t)r.lg << 6 |
+                                                         (lv[l].top ? 1u << 9 : 0u) |
+                                                         (uint32_t)(bars - seen[w]) << 16));
+          seen[w] = bars;
+          if (!lv[l].narrow) w = (w + 1) % nw;
+        }
+      }
+      ++bars;  // the pass ends with one
+      for (int w = 0; w < nw; ++w) {
+        wptr.push_back((int)out.size());
+        out.insert(out.end(), per[w].begin(), per[w].end());
+        out.push_back(make_uint2(0, (uint32_t)(bars - seen[w]) << 16));
+      }
+      wptr.push_back((int)out.size());
+      lv.clear();
+    };
+    auto by_length = [&](std::vector<int>& items, auto&& len) {
+      if (!same)
+        std::stable_sort(items.begin(), items.end(), [&](int x, int z) { return len(x) > len(z); });
+      std::vector<int> l;
+      for (int i : items) l.push_back(len(i));
+      return l;
+    };
+    for (int l = 0; l < nlev; ++l) {
+      const int l1 = l == L0 ? nlev : l + 1, a0 = (int)wact.size();
+      std::vector<int> items;
+      for (int t = ftask_ptr[l]; t < ftask_ptr[l1]; ++t)
+        if (ftask[t].w || ftask[t].z > ftask[t].y) items.push_back(t);
+      const auto len = by_length(items, [&](int t) { return ftask[t].z - ftask[t].y; });
+      for (int t : items)
+        wact.push_back(make_uint4((uint32_t)ftask[t].y,
+                                  (uint32_t)(ftask[t].z - ftask[t].y) | ((uint32_t)ftask[t].w << 31),
+                                  (uint32_t)ftask[t].x, 0));
+      add_level(a0, len, md_fac[l], false);
+      if (l1 == nlev) break;
+    }
+    rounds(wfr);
+    auto columns = [&](int c0, int c1, uint8_t md, bool back, bool top) {
+      std::vector<int> items;
+      for (int j = c0; j < c1; ++j) items.push_back(j);
+      const auto len = by_length(items, [&](int j) {
+        return back ? colptr[j + 1] - colptr[j] - 1 : fitem[j].z - fitem[j].y;
+      });
+      auto& out = back ? wcb : wcf;
+      const int a0 = (int)out.size();
+      for (size_t q = 0; q < items.size(); ++q) {
+        const int j = items[q];
+        out.push_back(make_uint4((uint32_t)fitem[j].y, (uint32_t)len[q], (uint32_t)colptr[j],
+                                 (uint32_t)j));
+      }
+      add_level(a0, len, md, top);
+    };
+    for (int l = 0; l <= std::min(L0, nlev - 1); ++l)
+      columns(levptr[l], l == L0 ? Nj : levptr[l + 1], md_fwd[l], false, l == L0);
+    rounds(wcr);
+    for (int l = L0 - 1; l >= 0; --l) columns(levptr[l], levptr[l + 1], md_bwd[l], true, false);
+    rounds(wbr);
+    for (size_t q = 0; q + 2 < fpair.size(); q += 3)
+      wterm.push_back(make_uint4((uint32_t)fpair[q], (uint32_t)fpair[q + 1],
+                                 (uint32_t)fpair[q + 2], 0));
+    for (auto* v : {&wact, &wterm, &wcf, &wcb})
+      if (v->empty()) v->push_back(make_uint4(0, 0, 0, 0));
+  };
+  struct TabOff { int sp, fp, cp, ri, lp, rp, re, md, ip, is, in, e1, e2, pp, pl, ps, fl, ds, ac, te, co, cb, rf, rc, rb, r3; };
   auto pack = [&](auto tag, Blob& sb, TabOff& o) {
     using S = decltype(tag);
     constexpr bool W32 = sizeof(S) == 4;
@@ -678,6 +795,11 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     o.rp = sadd(rp); o.re = sadd(re); o.md = sadd(s_md); o.ip = sadd(s_ip); o.is = sadd(s_is);
     o.in = sadd(s_in); o.e1 = sadd(s_e1); o.e2 = sadd(s_e2); o.pp = sadd(s_pp); o.pl = sadd(s_pl);
     o.ps = sadd(ps); o.fl = sadd(fl); o.ds = sadd(ds);
+    if constexpr (W32) {
+      o.ac = sadd(wact); o.te = sadd(wterm); o.co = sadd(wcf); o.cb = sadd(wcb);
+      o.rf = sadd(wfr); o.rc = sadd(wcr); o.rb = sadd(wbr);
+      o.r3 = sadd(wptr);
+    }
     sb.bytes.resize((sb.bytes.size() + 15) / 16 * 16);
   };
   const bool fits16 = nnzL < 65535 && (int)fpair.size() / 3 < 65536 &&
@@ -693,15 +815,17 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
   TabOff to{};
   if (net->layout < WDS_LAYOUT_AUTO || net->layout > WDS_LAYOUT_GLOBAL)
     return fail(WDS_E_ARG, "wds_plan: unknown layout");
-  bool wide = !fits16 || net->layout == WDS_LAYOUT_GLOBAL;
-  if (!wide) {
+  bool small_fits = false;
+  if (fits16) {
     pack(uint16_t{}, sblob, to);
-    wide = sblob.bytes.size() + state_bytes > 227 * 1024;
+    small_fits = sblob.bytes.size() + state_bytes <= 227 * 1024;
   }
+  const bool wide = !small_fits || net->layout == WDS_LAYOUT_GLOBAL;
   if (wide && net->layout == WDS_LAYOUT_SHARED)
     return fail(WDS_E_UNSUPPORTED, "wds_plan: the network's tables and state exceed shared "
                                    "memory (layout WDS_LAYOUT_SHARED)");
   if (wide) {
+    large_tables(small_fits);
     sblob = Blob();
     pack(uint32_t{}, sblob, to);
   }
@@ -788,6 +912,8 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
   d.o_inc = to.in; d.o_e1 = to.e1; d.o_e2 = to.e2; d.o_pptr = to.pp; d.o_plink = to.pl;
   d.o_pslot = to.ps; d.o_fill = to.fl; d.o_dslot = to.ds;
   d.L0 = L0; d.cT = cT; d.nT = nT;
+  d.o_act = to.ac; d.o_term = to.te; d.o_colf = to.co; d.o_colb = to.cb;
+  d.o_frnd = to.rf; d.o_crnd = to.rc; d.o_brnd = to.rb; d.o_rptr3 = to.r3;
 #undef P_
   d.hexp = net->hexp; d.qexp = net->qexp; d.rqtol = net->rqtol; d.htol = net->htol;
   d.qtol = net->qtol; d.ucf_flow = net->ucf_flow; d.ucf_head = net->ucf_head;
