@@ -30,8 +30,6 @@ __host__ __device__ constexpr int top_ld(int nT) { return (nT + 1) & ~1; }
 struct DevNet {
   int N, L, Nj, Nf, nnzL, nlev, npcv, ntl, npairs, nfill, nxf, nftask, nfpair;
   // links [L]
-  const int* e1;
-  const int* e2;
   const int8_t* kind;
   const uint8_t* flags;
   const int8_t* status0;
@@ -55,9 +53,6 @@ struct DevNet {
   // junctions, elimination order [Nj]
   const int* jnode;       // node index
   const double* el;       // elevation
-  const int* inc_ptr;     // [Nj+1]
-  const int* inc_split;   // [Nj] first n2-side entry
-  const int* inc;         // link index of each incidence entry
   const int* xf_node;     // [nxf] junction of each Xflow slot
   const int* cb_ptr;      // [Nj+1] pcv valves whose downstream node is p
   const int* cb_idx;
@@ -66,22 +61,6 @@ struct DevNet {
   const int* finc_ptr;    // [Nf+1]
   const int* finc_split;  // [Nf]
   const int* finc;
-  // off-diagonal entries of A
-  const int* pair_ptr;    // [npairs+1]
-  const int* pair_link;
-  const int* pair_slot;   // [npairs]
-  const int* fill_slot;   // [nfill]
-  // symbolic structure of L (column-major, diagonal first)
-  const int* colptr;      // [Nj+1]
-  const int* rowidx;      // [nnzL]
-  const int* levptr;      // [nlev+1]
-  const int* levcol;      // [Nj]
-  const int* ftask_ptr;   // [nlev+1]
-  const int4* ftask;      // {slot, pair_begin, pair_end, is_diag}
-  const int* fpair;       // [3*nfpair] {s1, s2, diag slot of k}
-  const int4* fitem;      // [Nj] level order: {j, row entry begin, end, diag slot}
-  const int4* bitem;      // [Nj] level order: {j, colptr[j], colptr[j+1], 0}
-  const int2* rent;       // row entries {slot of L_jk, k}, level order
   // status-machine PRVs [npcv]
   const int* pcv_link;
   const int* pcv_j1;

@@ -15,9 +15,9 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <map>
-#include <set>
+#include <functional>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "wds_internal.h"
@@ -47,36 +47,43 @@ std::vector<int> min_degree(int n, std::vector<std::vector<int>> adj) {
   std::vector<int> deg(n), lev(n, 0), order;
   order.reserve(n);
   std::vector<char> alive(n, 1);
-  std::set<std::pair<int, int>> pq;
-  auto key = [&](int i) { return std::make_pair(2 * deg[i] + lev[i], i); };
+  // heap of key << 32 | row; an entry whose key is no longer the row's is stale
+  std::vector<uint64_t> heap;
+  auto key = [&](int i) { return (uint64_t)(2 * deg[i] + lev[i]) << 32 | (uint32_t)i; };
   for (int i = 0; i < n; ++i) {
     deg[i] = (int)adj[i].size();
-    pq.insert(key(i));
+    heap.push_back(key(i));
   }
-  std::vector<int> merged;
-  while (!pq.empty()) {
-    int v = pq.begin()->second;
-    pq.erase(pq.begin());
+  const std::greater<uint64_t> later;
+  std::make_heap(heap.begin(), heap.end(), later);
+  std::vector<int> nb, nu;
+  while (!heap.empty()) {
+    std::pop_heap(heap.begin(), heap.end(), later);
+    const uint64_t top = heap.back();
+    heap.pop_back();
+    const int v = (int)(uint32_t)top;
+    if (!alive[v] || top != key(v)) continue;
     alive[v] = 0;
     order.push_back(v);
-    std::vector<int> nb;
-    for (int u : adj[v])
-      if (alive[u]) nb.push_back(u);
+    nb.swap(adj[v]);  // an eliminated row is in no list
     for (int u : nb) {
-      pq.erase(key(u));
-      merged.clear();
-      std::set_union(adj[u].begin(), adj[u].end(), nb.begin(), nb.end(),
-                     std::back_inserter(merged));
-      std::vector<int> nu;
-      nu.reserve(merged.size());
-      for (int w : merged)
-        if (w != u && alive[w]) nu.push_back(w);
-      adj[u].swap(nu);
-      deg[u] = (int)adj[u].size();
+      nu.clear();
+      const std::vector<int>& au = adj[u];
+      size_t x = 0, y = 0;  // the union of au and nb without u and v
+      while (x < au.size() || y < nb.size()) {
+        int w;
+        if (y == nb.size() || (x < au.size() && au[x] < nb[y])) w = au[x++];
+        else if (x == au.size() || nb[y] < au[x]) w = nb[y++];
+        else { w = au[x++]; ++y; }
+        if (w != u && w != v) nu.push_back(w);
+      }
+      adj[u].assign(nu.begin(), nu.end());
+      deg[u] = (int)nu.size();
       lev[u] = std::max(lev[u], lev[v] + 1);
-      pq.insert(key(u));
+      heap.push_back(key(u));
+      std::push_heap(heap.begin(), heap.end(), later);
     }
-    adj[v].clear();
+    std::vector<int>().swap(adj[v]);
   }
   return order;
 }
@@ -310,45 +317,53 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     if (it == e || *it != i) return -1;
     return (int)(it - rowidx.begin());
   };
-  // row lists: rows[i] = { k < i : i in struct(k) } ascending; a top row keeps
-  // only its entries in the columns below the top block
-  std::vector<std::vector<int>> rows(Nj);
-  for (int k = 0; k < Nj; ++k)
-    for (int i : cstruct[k])
-      if (i < cT || k < cT) rows[i].push_back(k);
-  // forward-substitution items in level order: {j, first row entry, end, diag slot};
-  // row entries {slot of L_jk, k} stored contiguously in the same order
+  // forward-substitution rows in level order, {j, first row entry, end, diag
+  // slot}, with the entries {slot of L_jk, k}, k ascending; a top row keeps only
+  // its entries in the columns below the top block
   std::vector<int2> rent;
-  std::vector<int4> fitem(Nj), bitem(Nj);
-  for (int t = 0; t < Nj; ++t) {
-    int j = levcol[t];
-    int e0 = (int)rent.size();
-    for (int k : rows[j]) rent.push_back(make_int2(slot(j, k), k));
-    fitem[t] = make_int4(j, e0, (int)rent.size(), colptr[j]);
-    bitem[t] = make_int4(j, colptr[j], colptr[j + 1], 0);
+  std::vector<int4> fitem(Nj);
+  {
+    std::vector<int> pos(Nj + 1, 0);
+    for (int k = 0; k < cT; ++k)
+      for (int e = colptr[k] + 1; e < colptr[k + 1]; ++e) ++pos[rowidx[e] + 1];
+    for (int j = 0; j < Nj; ++j) {
+      pos[j + 1] += pos[j];
+      fitem[j] = make_int4(j, pos[j], pos[j + 1], colptr[j]);
+    }
+    rent.resize(std::max(pos[Nj], 1), make_int2(0, 0));
+    for (int k = 0; k < cT; ++k)
+      for (int e = colptr[k] + 1; e < colptr[k + 1]; ++e)
+        rent[pos[rowidx[e]]++] = make_int2(e, k);
   }
-  if (rent.empty()) rent.push_back(make_int2(0, 0));
-  // factor tasks by level
+  // factor tasks by level, one per entry of L in slot order: {slot, first
+  // update, end, diagonal below the top block}; an update of L_ij is {L_ik,
+  // L_jk, 1/D_k} for each k of row j with i in column k (k ascending)
   std::vector<int> ftask_ptr(nlev + 1, 0), fpair;
-  std::vector<int4> ftask;
-  for (int l = 0; l < nlev; ++l) {
-    for (int t = levptr[l]; t < levptr[l + 1]; ++t) {
-      int j = levcol[t];
-      for (int e = colptr[j]; e < colptr[j + 1]; ++e) {
-        int i = rowidx[e];
-        int pb = (int)fpair.size() / 3;
-        for (int k : rows[j]) {
-          int sik = slot(i, k);
-          if (sik < 0) continue;
-          fpair.push_back(sik);
-          fpair.push_back(slot(j, k));
-          fpair.push_back(colptr[k]);
+  std::vector<int4> ftask(nnzL);
+  {
+    std::vector<int> loc(Nj), at;
+    for (int j = 0; j < Nj; ++j) {
+      const int c0 = colptr[j], c1 = colptr[j + 1], f0 = (int)(fpair.size() / 3);
+      at.assign(c1 - c0 + 1, 0);
+      for (int e = c0; e < c1; ++e) loc[rowidx[e]] = e - c0;
+      for (int t = fitem[j].y; t < fitem[j].z; ++t)
+        for (int q = rent[t].x; q < colptr[rent[t].y + 1]; ++q) ++at[loc[rowidx[q]] + 1];
+      for (int e = c0; e < c1; ++e) {
+        at[e - c0 + 1] += at[e - c0];
+        ftask[e] = make_int4(e, f0 + at[e - c0], f0 + at[e - c0 + 1], (e == c0 && j < cT) ? 1 : 0);
+      }
+      fpair.resize(fpair.size() + 3 * (size_t)at[c1 - c0]);
+      for (int t = fitem[j].y; t < fitem[j].z; ++t) {
+        const int k = rent[t].y;
+        for (int q = rent[t].x; q < colptr[k + 1]; ++q) {
+          int* f = &fpair[3 * (size_t)(f0 + at[loc[rowidx[q]]]++)];
+          f[0] = q;
+          f[1] = rent[t].x;
+          f[2] = colptr[k];
         }
-        int pe = (int)fpair.size() / 3;
-        ftask.push_back(make_int4(e, pb, pe, (i == j && j < cT) ? 1 : 0));
       }
     }
-    ftask_ptr[l + 1] = (int)ftask.size();
+    for (int l = 0; l < nlev; ++l) ftask_ptr[l + 1] = colptr[levptr[l + 1]];
   }
   // Execution mode per level and operation, one byte: bits 0-2 = log2 of the
   // lane-group size G (each item's dot product is spread over G lanes and
@@ -381,7 +396,7 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     for (int t = ftask_ptr[l]; t < ftask_ptr[l1]; ++t) mf = std::max(mf, ftask[t].z - ftask[t].y);
     for (int t = levptr[l]; t < levptr[l1]; ++t) {
       int j = levcol[t];
-      mr = std::max(mr, (int)rows[j].size());
+      mr = std::max(mr, fitem[j].z - fitem[j].y);
       mc = std::max(mc, colptr[j + 1] - colptr[j] - 1);
     }
     md_fac[l] = pick_mode(ftask_ptr[l1] - ftask_ptr[l], mf);
@@ -419,20 +434,25 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     finc.insert(finc.end(), finc2[f].begin(), finc2[f].end());
     finc_ptr[f + 1] = (int)finc.size();
   }
-  std::map<std::pair<int, int>, std::vector<int>> pairs;
+  struct Pair { int hi, lo, k; };
+  std::vector<Pair> pairs;
   for (int k = 0; k < L; ++k)
     if (e1[k] >= 0 && e2[k] >= 0 && e1[k] != e2[k])
-      pairs[{std::max(e1[k], e2[k]), std::min(e1[k], e2[k])}].push_back(k);
-  std::vector<int> pair_ptr(1, 0), pair_link, pair_slot;
+      pairs.push_back({std::max(e1[k], e2[k]), std::min(e1[k], e2[k]), k});
+  std::sort(pairs.begin(), pairs.end(), [](const Pair& a, const Pair& b) {
+    return std::tie(a.hi, a.lo, a.k) < std::tie(b.hi, b.lo, b.k);
+  });
+  std::vector<int> pair_ptr(1, 0), pair_link, pair_slot, slot_of_link(L, 0);
   std::vector<char> is_a(nnzL, 0);
-  std::map<std::pair<int, int>, int> pair_slot_of;
-  for (auto& kv : pairs) {
-    int s = slot(kv.first.first, kv.first.second);
+  for (size_t a = 0; a < pairs.size(); ++a) {
+    const int s = slot(pairs[a].hi, pairs[a].lo);
     if (s < 0) return fail(WDS_E_ARG, "wds_plan: internal error (pair outside pattern)");
+    slot_of_link[pairs[a].k] = s;
+    pair_link.push_back(pairs[a].k);
+    if (a + 1 < pairs.size() && pairs[a + 1].hi == pairs[a].hi && pairs[a + 1].lo == pairs[a].lo)
+      continue;
     is_a[s] = 1;
-    pair_slot_of[kv.first] = s;
     pair_slot.push_back(s);
-    pair_link.insert(pair_link.end(), kv.second.begin(), kv.second.end());
     pair_ptr.push_back((int)pair_link.size());
   }
   std::vector<int> fill_slot;
@@ -460,7 +480,7 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     pcv_jo.push_back(jo);
     pcv_sgn.push_back(psv ? -1.0 : 1.0);
     pcv_psv.push_back(psv ? 1 : 0);
-    pcv_off.push_back(pair_slot_of[{std::max(e1[k], e2[k]), std::min(e1[k], e2[k])}]);
+    pcv_off.push_back(slot_of_link[k]);
     if (node_xf[jc] < 0) {
       node_xf[jc] = nxf++;
       xf_node.push_back(jc);
@@ -483,7 +503,7 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     fcv_link.push_back(k);
     fcv_j1.push_back(e1[k]);
     fcv_j2.push_back(e2[k]);
-    fcv_off.push_back(pair_slot_of[{std::max(e1[k], e2[k]), std::min(e1[k], e2[k])}]);
+    fcv_off.push_back(slot_of_link[k]);
     fcv_xf1.push_back(node_xf[e1[k]]);
     fcv_xf2.push_back(node_xf[e2[k]]);
     fcv_qs.push_back(net->prv_hset[k]);
@@ -566,8 +586,7 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     for (auto& r : rent) ok = ok && in(r.x, 0, nnzL) && in(r.y, 0, Nj);
     for (int t = 0; t < Nj; ++t)
       ok = ok && in(fitem[t].x, 0, Nj) && fitem[t].y >= 0 && fitem[t].y <= fitem[t].z &&
-           fitem[t].z <= (int)rent.size() && in(fitem[t].w, 0, nnzL) && in(bitem[t].x, 0, Nj) &&
-           bitem[t].y >= 0 && bitem[t].y < bitem[t].z && bitem[t].z <= nnzL;
+           fitem[t].z <= (int)rent.size() && in(fitem[t].w, 0, nnzL);
     for (int v : dsl) ok = ok && (v == -1 || in(v, colptr[cT], nnzL));
     ok = ok && nT >= 0 && nT <= WDS_TOP_MAX;
     for (int v : cb_idx) ok = ok && in(v, 0, std::max(npcv, 1));
@@ -832,32 +851,25 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
   std::vector<unsigned char> stab_bytes = sblob.bytes;
   // ---- upload
   Blob blob;
-  size_t o_e1 = blob.add(e1), o_e2 = blob.add(e2), o_kind = blob.add(kind), o_flags = blob.add(flags),
-         o_st0 = blob.add(st0), o_ptype = blob.add(ptype), o_km = blob.add(km),
-         o_kmt = blob.add(km_tcv), o_q0 = blob.add(q_init), o_ph0 = blob.add(ph0),
-         o_pr = blob.add(pr), o_pn = blob.add(pn), o_psp = blob.add(psp), o_phm = blob.add(phm),
+  size_t o_kind = blob.add(kind), o_flags = blob.add(flags), o_st0 = blob.add(st0),
+         o_ptype = blob.add(ptype), o_km = blob.add(km), o_kmt = blob.add(km_tcv),
+         o_q0 = blob.add(q_init), o_ph0 = blob.add(ph0), o_pr = blob.add(pr),
+         o_pn = blob.add(pn), o_psp = blob.add(psp), o_phm = blob.add(phm),
          o_cptr = blob.add(cptr), o_cx = blob.add(cx), o_cy = blob.add(cy),
          o_ltl = blob.add(link_tl), o_lpcv = blob.add(link_pcv), o_jn = blob.add(jn),
-         o_el = blob.add(el), o_incp = blob.add(inc_ptr), o_incs = blob.add(inc_split),
-         o_inc = blob.add(inc), o_nxf = blob.add(xf_node), o_cbp = blob.add(cb_ptr),
+         o_el = blob.add(el), o_nxf = blob.add(xf_node), o_cbp = blob.add(cb_ptr),
          o_cbi = blob.add(cb_idx), o_fn = blob.add(fnodes), o_fincp = blob.add(finc_ptr),
-         o_fincs = blob.add(finc_split), o_finc = blob.add(finc), o_pp = blob.add(pair_ptr),
-         o_pl = blob.add(pair_link), o_ps = blob.add(pair_slot), o_fs = blob.add(fill_slot),
-         o_cp = blob.add(colptr), o_ri = blob.add(rowidx), o_lp = blob.add(levptr),
-         o_lc = blob.add(levcol), o_ftp = blob.add(ftask_ptr), o_ft = blob.add(ftask),
-         o_fp = blob.add(fpair), o_rent = blob.add(rent), o_fit = blob.add(fitem),
-         o_bit = blob.add(bitem),
-         o_pcl = blob.add(pcv_link), o_pj1 = blob.add(pcv_j1), o_pj2 = blob.add(pcv_j2),
-         o_poff = blob.add(pcv_off), o_pxf = blob.add(pcv_xf), o_phs = blob.add(pcv_hset),
-         o_pkm = blob.add(pcv_km), o_tll = blob.add(tl_link), o_tlt = blob.add(tl_tank),
-         o_tlo = blob.add(tl_other), o_tlq = blob.add(tl_qsign), o_tlx = blob.add(tl_hmax),
-         o_tln = blob.add(tl_hmin), o_tlf = blob.add(tl_flags), o_stab = blob.add(stab_bytes),
-         o_lpu = blob.add(link_pump), o_phu = blob.add(phu), o_lfc = blob.add(link_fcv),
-         o_fcl = blob.add(fcv_link), o_fj1 = blob.add(fcv_j1), o_fj2 = blob.add(fcv_j2),
-         o_fof = blob.add(fcv_off), o_fx1 = blob.add(fcv_xf1), o_fx2 = blob.add(fcv_xf2),
-         o_fqs = blob.add(fcv_qs), o_fkm = blob.add(fcv_km), o_vord = blob.add(vord),
-         o_pjc = blob.add(pcv_jc), o_pjo = blob.add(pcv_jo), o_psg = blob.add(pcv_sgn),
-         o_pps = blob.add(pcv_psv);
+         o_fincs = blob.add(finc_split), o_finc = blob.add(finc), o_pcl = blob.add(pcv_link),
+         o_pj1 = blob.add(pcv_j1), o_pj2 = blob.add(pcv_j2), o_poff = blob.add(pcv_off),
+         o_pxf = blob.add(pcv_xf), o_phs = blob.add(pcv_hset), o_pkm = blob.add(pcv_km),
+         o_tll = blob.add(tl_link), o_tlt = blob.add(tl_tank), o_tlo = blob.add(tl_other),
+         o_tlq = blob.add(tl_qsign), o_tlx = blob.add(tl_hmax), o_tln = blob.add(tl_hmin),
+         o_tlf = blob.add(tl_flags), o_stab = blob.add(stab_bytes), o_lpu = blob.add(link_pump),
+         o_phu = blob.add(phu), o_lfc = blob.add(link_fcv), o_fcl = blob.add(fcv_link),
+         o_fj1 = blob.add(fcv_j1), o_fj2 = blob.add(fcv_j2), o_fof = blob.add(fcv_off),
+         o_fx1 = blob.add(fcv_xf1), o_fx2 = blob.add(fcv_xf2), o_fqs = blob.add(fcv_qs),
+         o_fkm = blob.add(fcv_km), o_vord = blob.add(vord), o_pjc = blob.add(pcv_jc),
+         o_pjo = blob.add(pcv_jo), o_psg = blob.add(pcv_sgn), o_pps = blob.add(pcv_psv);
   WdsPlan* plan = new WdsPlan();
   if (cudaMalloc(&plan->dtab, blob.bytes.size()) != cudaSuccess) {
     delete plan;
@@ -875,7 +887,7 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
   d.N = N; d.L = L; d.Nj = Nj; d.Nf = Nf; d.nnzL = nnzL; d.nlev = nlev; d.npcv = npcv;
   d.ntl = ntl; d.npairs = (int)pair_slot.size(); d.nfill = (int)fill_slot.size(); d.nxf = nxf;
   d.nftask = (int)ftask.size(); d.nfpair = (int)fpair.size() / 3;
-  d.e1 = P_(int, o_e1); d.e2 = P_(int, o_e2); d.kind = P_(int8_t, o_kind);
+  d.kind = P_(int8_t, o_kind);
   d.flags = P_(uint8_t, o_flags); d.status0 = P_(int8_t, o_st0); d.ptype = P_(int8_t, o_ptype);
   d.km = P_(double, o_km); d.km_tcv = P_(double, o_kmt); d.q_init = P_(double, o_q0);
   d.ph0 = P_(double, o_ph0); d.pr = P_(double, o_pr); d.pn = P_(double, o_pn);
@@ -889,14 +901,9 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
   d.pcv_psv = P_(int, o_pps);
   d.cx = P_(double, o_cx); d.cy = P_(double, o_cy); d.link_tl = P_(int, o_ltl);
   d.link_pcv = P_(int, o_lpcv); d.jnode = P_(int, o_jn); d.el = P_(double, o_el);
-  d.inc_ptr = P_(int, o_incp); d.inc_split = P_(int, o_incs); d.inc = P_(int, o_inc);
   d.xf_node = P_(int, o_nxf); d.cb_ptr = P_(int, o_cbp); d.cb_idx = P_(int, o_cbi);
   d.fnode = P_(int, o_fn); d.finc_ptr = P_(int, o_fincp); d.finc_split = P_(int, o_fincs);
-  d.finc = P_(int, o_finc); d.pair_ptr = P_(int, o_pp); d.pair_link = P_(int, o_pl);
-  d.pair_slot = P_(int, o_ps); d.fill_slot = P_(int, o_fs); d.colptr = P_(int, o_cp);
-  d.rowidx = P_(int, o_ri); d.levptr = P_(int, o_lp); d.levcol = P_(int, o_lc);
-  d.ftask_ptr = P_(int, o_ftp); d.ftask = P_(int4, o_ft); d.fpair = P_(int, o_fp);
-  d.rent = P_(int2, o_rent); d.fitem = P_(int4, o_fit); d.bitem = P_(int4, o_bit);
+  d.finc = P_(int, o_finc);
   d.pcv_link = P_(int, o_pcl); d.pcv_j1 = P_(int, o_pj1); d.pcv_j2 = P_(int, o_pj2);
   d.pcv_off = P_(int, o_poff); d.pcv_xf = P_(int, o_pxf); d.pcv_hset = P_(double, o_phs);
   d.pcv_km = P_(double, o_pkm); d.tl_link = P_(int, o_tll); d.tl_tank = P_(int, o_tlt);
