@@ -97,6 +97,7 @@ struct DevNet {
   const double* tl_hmin;
   const uint8_t* tl_flags;
   double hexp, qexp, rqtol, htol, qtol, ucf_flow, ucf_head;
+  double rhexp;  // 1 / hexp
   int checkfreq, maxcheck, extra_iter;
   // compact 16-bit copy of the hot schedule tables, staged into shared memory
   // once per CTA (see STabOff)

@@ -922,6 +922,7 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
   d.o_act = to.ac; d.o_term = to.te; d.o_colf = to.co; d.o_colb = to.cb;
   d.o_frnd = to.rf; d.o_crnd = to.rc; d.o_brnd = to.rb; d.o_rptr3 = to.r3;
 #undef P_
+  d.rhexp = 1.0 / net->hexp;
   d.hexp = net->hexp; d.qexp = net->qexp; d.rqtol = net->rqtol; d.htol = net->htol;
   d.qtol = net->qtol; d.ucf_flow = net->ucf_flow; d.ucf_head = net->ucf_head;
   d.checkfreq = net->checkfreq; d.maxcheck = net->maxcheck; d.extra_iter = net->extra_iter;
