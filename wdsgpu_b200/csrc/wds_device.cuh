@@ -73,8 +73,13 @@ struct Sh {
 template <class Slot>
 struct TabT {
   static constexpr bool kWide = sizeof(Slot) == 4;
-  const uint32_t* spair;      // per slot: begin | count << 16 | diagonal << 31 (wide: 2 words, begin and count | diagonal << 31)
-  const Slot* fpair;          // [3 * terms] {slot L_ik, slot L_jk, slot 1/D_k}
+  const uint16_t* kf;         // [L] kind | flags << 8 (WDS_F_*, kStatusLink, kMinorLoss)
+  const ValveRec* vrec;       // status-machine valves in the order of the valve pass
+  // small networks: first term of the update list of every entry of L | its
+  // diagonal flag << 15, one more at the end; the terms {slot L_ik, slot L_jk,
+  // slot 1/D_k}
+  const uint16_t* spair;
+  const uint16_t* fpair;
   const Slot* colptr;         // [Nj+1]
   const uint16_t* rowidx;     // [nnzL]
   const uint16_t* levptr;     // [nlev+1] columns of a level (columns numbered in level order)
@@ -106,17 +111,10 @@ struct TabT {
 
   // update list of the entry in `slot`: first term, term count, diagonal flag
   __device__ __forceinline__ void sp(int slot, int& pb, int& cnt, bool& diag) const {
-    if constexpr (kWide) {
-      const uint2 w = reinterpret_cast<const uint2*>(spair)[slot];
-      pb = (int)w.x;
-      cnt = (int)(w.y & 0x7fffffffu);
-      diag = (w.y >> 31) != 0;
-    } else {
-      const uint32_t w = spair[slot];
-      pb = (int)(w & 0xffffu);
-      cnt = (int)((w >> 16) & 0x7fffu);
-      diag = (w >> 31) != 0;
-    }
+    const int w = spair[slot], z = spair[slot + 1];
+    pb = w & 0x7fff;
+    cnt = (z & 0x7fff) - pb;
+    diag = (w >> 15) != 0;
   }
   // row-list entry e: slot of L_jk and column k
   __device__ __forceinline__ void re(int e, int& slot, int& k) const {
@@ -140,8 +138,10 @@ __device__ TB tab_view(const DevNet& n, const unsigned char* b) {
   using Slot = typename std::remove_pointer<decltype(TB::colptr)>::type;
   using S = typename std::remove_const<Slot>::type;
   TB t;
-  t.spair = (const uint32_t*)(b + n.o_spair);
-  t.fpair = (const S*)(b + n.o_fpair);
+  t.kf = (const uint16_t*)(b + n.o_kf);
+  t.vrec = (const ValveRec*)(b + n.o_vrec);
+  t.spair = (const uint16_t*)(b + n.o_spair);
+  t.fpair = (const uint16_t*)(b + n.o_fpair);
   t.colptr = (const S*)(b + n.o_colptr);
   t.rowidx = (const uint16_t*)(b + n.o_rowidx);
   t.levptr = (const uint16_t*)(b + n.o_levptr);
@@ -496,9 +496,11 @@ __device__ __forceinline__ void prv_open(const DevNet& n, int i, double qk, int 
 // Link coefficients of the headloss stage (dgga/solver.py:2923-2956).
 // `adj` selects the adjoint/polish variant in which a status-machine PRV
 // takes its valve coefficients directly (autodiff.py:838-847).
-__device__ __forceinline__ void link_coef(const DevNet& n, const PumpTh& th, int k, double q,
-                                          int s, double r, bool adj, double& P, double& Y) {
-  const int kd = n.kind[k];
+// `kf` is the link's entry of the table of that name.
+__device__ __forceinline__ void link_coef(const DevNet& n, const PumpTh& th, int k, uint32_t kf,
+                                          double q, int s, double r, bool adj, double& P,
+                                          double& Y) {
+  const int kd = (int)(kf & 0xff);
   if (kd == WDS_KIND_FCV) {  // the valve pass fills the GGA coefficients
     if (!adj) {
       P = 0.0;
@@ -523,13 +525,15 @@ __device__ __forceinline__ void link_coef(const DevNet& n, const PumpTh& th, int
     }
     return;
   }
-  if (s <= WDS_CLOSED || zero_speed(n, th, k, kd)) {
+  const bool still = th.own_sp() ? (kd == WDS_KIND_PUMP && th.sp(k) == 0.0)
+                                 : (kf >> 8 & WDS_F_ZERO_SPEED) != 0;  // as zero_speed
+  if (s <= WDS_CLOSED || still) {
     P = 1.0 / kCBIG;
     Y = q;
     return;
   }
   if (kd <= WDS_KIND_CVPIPE)
-    pipe_coef(n, q, r, n.km[k], P, Y);
+    pipe_coef(n, q, r, kf >> 8 & kMinorLoss ? n.km[k] : 0.0, P, Y);
   else if (kd == WDS_KIND_TCV)
     valve_open(n, q, n.km_tcv[k], P, Y);
   else if (kd == WDS_KIND_PRV_FIXED)
@@ -1351,20 +1355,21 @@ __device__ void link_pass(const DevNet& n, const PumpTh& th, const TB& T, const 
   double qn = k < n.L ? s.q[k] : 0.0, rn = k < n.L ? rrow[k] : 0.0;
   for (; k < n.L; k += NT) {
     const double qk = qn, rk = rn;
+    const uint32_t kf = T.kf[k];
     const int kn = k + NT;
     if (kn < n.L) {
       qn = s.q[kn];
       rn = rrow[kn];
     }
     double P, Y;
-    link_coef(n, th, k, qk, s.S[k], rk, false, P, Y);
+    link_coef(n, th, k, kf, qk, s.S[k], rk, false, P, Y);
     s.P[k] = P;
     s.Y[k] = Y;
     const int c1 = T.e1[k], c2 = T.e2[k];
     double z = Y - qk;
     if (c2 < 0 && c1 >= 0) z += P * s.hf[-c2 - 1];
     if (c1 < 0 && c2 >= 0) z -= P * s.hf[-c1 - 1];
-    const int kd = n.kind[k];
+    const int kd = (int)(kf & 0xff);
     Z[k] = kd == WDS_KIND_PRV || kd == WDS_KIND_PSV || kd == WDS_KIND_FCV ? 0.0 : z;
   }
   for (int es = tid; es < s.flag[2]; es += NT) {
@@ -1418,63 +1423,79 @@ __device__ void assemble_gga(const DevNet& n, const TB& T, const Sh& s, const do
     wp<FT>(s)[T.pslot[t]] = (FT)v;
   }
   for (int t = tid; t < n.nfill; t += NT) wp<FT>(s)[T.fill[t]] = FT(0);
+  // valvecoeffs after nodecoeffs, in valve order: a lane of the last warp (the
+  // fewest junctions) per valve loads its flow and status and forms its
+  // coefficients before the barrier, all valves at once, and the lanes then
+  // take their turns at what depends on the order.
+  const int nv = n.npcv + n.nfcv, lane = threadIdx.x & 31;
+  if (nv == 0) {
+    gsync<NT>();
+    return;
+  }
+  const bool mine = tid >= NT - 32;
+  int o = 0, k = 0, j1 = 0, j2 = 0, off = 0, jc = 0, jo = 0, x1 = 0, x2 = 0;
+  double qk = 0.0, pk = 0.0, yk = 0.0, set = 0.0, sg = 0.0;
+  bool act = false;
+  auto fetch = [&](int v) {
+    const ValveRec& r = T.vrec[v];
+    k = r.k;
+    qk = s.q[k];
+    o = r.fcv;
+    j1 = r.j1;
+    j2 = r.j2;
+    off = r.off;
+    x1 = r.x1;
+    x2 = r.x2;
+    jc = r.jc;
+    jo = r.jo;
+    set = r.set;
+    sg = r.sgn;
+    const int sk = s.S[k];
+    act = sk == WDS_ACTIVE;
+    if (o && act) {
+      pk = 1.0 / kCBIG;
+      yk = qk - set;
+    } else {
+      valve_state_coef(n, r.km, qk, sk, pk, yk);
+      if (!o) pk = pk * (act ? 0.0 : 1.0);  // as prv_open
+    }
+  };
+  if (mine && lane < nv) fetch(lane);
   gsync<NT>();
-  if (tid == 0) {  // valvecoeffs after nodecoeffs, in valve order
-    for (int v = 0; v < n.npcv + n.nfcv; ++v) {
-      const int o = n.vord[v];
-      if (o < 0) {  // FCV (fcvcoeff, hydcoeffs.c:1047-1097 as in dgga/solver.py:1665-1695)
-        const int f = -1 - o, k = n.fcv_link[f];
-        const double qk = s.q[k];
-        const int j1 = n.fcv_j1[f], j2 = n.fcv_j2[f];
-        FT* W = wp<FT>(s);
-        double pk, yk;
-        if (s.S[k] == WDS_ACTIVE) {
-          // the setting cuts the network: an outflow at n1, an inflow at n2
-          const double qs = n.fcv_qs[f];
-          if (n.fcv_xf1[f] >= 0) s.xf[n.fcv_xf1[f]] -= qs;
-          if (n.fcv_xf2[f] >= 0) s.xf[n.fcv_xf2[f]] += qs;
-          yk = qk - qs;
-          s.V0[j1] -= qs;
-          s.V0[j2] += qs;
-          pk = 1.0 / kCBIG;
+  if (mine) {
+    FT* W = wp<FT>(s);
+    for (int v = 0; v < nv; ++v) {
+      if (v > 0 && (v & 31) == 0 && v + lane < nv) fetch(v + lane);
+      if (lane == (v & 31)) {
+        double dy = yk - qk;
+        if (o) {  // FCV (fcvcoeff, hydcoeffs.c:1047-1097 as in dgga/solver.py:1665-1695)
+          if (act) {  // the setting cuts the network: an outflow at n1, an inflow at n2
+            if (x1 >= 0) s.xf[x1] -= set;
+            if (x2 >= 0) s.xf[x2] += set;
+            dy = -set;
+          }
         } else {
-          valve_state_coef(n, n.fcv_km[f], qk, s.S[k], pk, yk);
-          s.V0[j1] += yk - qk;
-          s.V0[j2] -= yk - qk;
+          // prvcoeff / psvcoeff (hydcoeffs.c:959-1044 as in dgga/solver.py:
+          // 862-903, 1647-1664): an ACTIVE valve holds the head of jc (PRV: n2,
+          // PSV: n1) by a CBIG penalty and reads the flow excess there
+          const double xfc = s.xf[x1];
+          if (act) {
+            dy = 0.0;
+            W[T.colptr[jc]] += (FT)kCBIG;
+            if (sg * xfc < 0.0) s.V0[jo] += xfc;
+            s.V0[jc] += set * kCBIG;
+            yk = qk + sg * xfc;
+          }
         }
-        W[n.fcv_off[f]] += (FT)(-pk);
+        W[off] += (FT)(-pk);
         W[T.colptr[j1]] += (FT)pk;
         W[T.colptr[j2]] += (FT)pk;
+        s.V0[j1] += dy;
+        s.V0[j2] -= dy;
         s.P[k] = pk;
         s.Y[k] = yk;
-        continue;
       }
-      const int i = o;
-      const int k = n.pcv_link[i];
-      const double qk = s.q[k];
-      const int sk = s.S[k];
-      const bool act = sk == WDS_ACTIVE;
-      double pna, yna;
-      prv_open(n, i, qk, sk, pna, yna);
-      const double mna = act ? 0.0 : 1.0, mact = act ? 1.0 : 0.0;
-      // prvcoeff / psvcoeff (hydcoeffs.c:959-1044 as in dgga/solver.py:
-      // 862-903, 1647-1664): an ACTIVE valve holds the head of jc (PRV: n2,
-      // PSV: n1) by a CBIG penalty and reads the flow excess there
-      const double xfc = s.xf[n.pcv_xf[i]], sg = n.pcv_sgn[i];
-      const double dy = (yna - qk) * mna;
-      const int j1 = n.pcv_j1[i], j2 = n.pcv_j2[i], jc = n.pcv_jc[i], jo = n.pcv_jo[i];
-      const double fo = (act && sg * xfc < 0.0) ? xfc : 0.0;
-      FT* W = wp<FT>(s);
-      W[n.pcv_off[i]] += (FT)(-pna);
-      W[T.colptr[j1]] += (FT)pna;
-      W[T.colptr[j2]] += (FT)pna;
-      W[T.colptr[jc]] += (FT)(kCBIG * mact);
-      s.V0[j1] += dy;
-      s.V0[j2] -= dy;
-      s.V0[jo] += fo;
-      s.V0[jc] += n.pcv_hset[i] * kCBIG * mact;
-      s.P[k] = pna;
-      s.Y[k] = act ? qk + sg * xfc : yna;
+      __syncwarp();
     }
   }
   gsync<NT>();
@@ -1511,17 +1532,27 @@ __device__ void assemble_reduced(const DevNet& n, const TB& T, const Sh& s) {
 // factor in use was formed with), `far` reports whether any of them moved
 // by more than tol, relative; their loads are issued before the
 // coefficients are formed.
-template <int NT>
-__device__ void adj_coeffs(const DevNet& n, const PumpTh& th, const Sh& s, const double* rrow,
+template <int NT, class TB>
+__device__ void adj_coeffs(const DevNet& n, const PumpTh& th, const TB& T, const Sh& s,
+                           const double* rrow,
                            const double* kerow, const double* Pf = nullptr,
                            const double* Ef = nullptr, double tol = 0.0,
                            bool* far = nullptr) {
   const int tid = gtid<NT>();
   bool fr = false;
-  for (int k = tid; k < n.L; k += NT) {
-    const double p0 = Pf ? Pf[k] : 0.0;
+  int k = tid;
+  double qn = 0.0, rn = 0.0, pn = 0.0;  // the next link's
+  auto fetch = [&](int i) {
+    qn = s.q[i];
+    rn = rrow[i];
+    pn = Pf ? Pf[i] : 0.0;
+  };
+  if (k < n.L) fetch(k);
+  for (; k < n.L; k += NT) {
+    const double qk = qn, rk = rn, p0 = pn;
+    if (k + NT < n.L) fetch(k + NT);
     double P, Y;
-    link_coef(n, th, k, s.q[k], s.S[k], rrow[k], true, P, Y);
+    link_coef(n, th, k, T.kf[k], qk, s.S[k], rk, true, P, Y);
     s.P[k] = P;
     s.Y[k] = Y;
     if (Pf) fr = fr || !(fabs(P - p0) <= tol * fabs(p0));
@@ -1715,27 +1746,37 @@ __host__ __device__ __forceinline__ Sh place_state(const DevNet& n, Take&& take)
   return s;
 }
 
-// The state at `base` (shared memory on the small-network layout).
+// The state at `base` (shared memory on the small-network layout).  The pieces
+// lie at offsets the plan computed, kernel parameters: a piece's address is one
+// addition wherever it is used, not a register held (or spilled) from the
+// start of the scenario on.
 __device__ __forceinline__ Sh carve(const DevNet& n, unsigned char* base) {
-  size_t o = 0;
-  return place_state(n, [&](size_t bytes) {
-    unsigned char* p = base + o;
-    o += al16(bytes);
-    return p;
+  int i = 0;
+  return place_state(n, [&](size_t) { return base + n.so[i++]; });
+}
+
+// The state of the large-network layout: a piece in shared memory at `sm`, or
+// (a negative offset) in the scenario's slice of the global workspace.
+__device__ __forceinline__ Sh carve_split(const DevNet& n, unsigned char* sm,
+                                          unsigned char* base) {
+  int i = 0;
+  return place_state(n, [&](size_t) {
+    const int o = n.so[i++];
+    return o >= 0 ? sm + o : base + ~o;
   });
 }
 
-// The state of the large-network layout: each piece in the n.sm_state bytes
-// of shared memory at `sm` while they last, else in the scenario's slice of
+// The offsets of the state's pieces: one after the other; on the large-network
+// layout each in the n.sm_state bytes of shared memory while they last, else in
 // the global workspace.
-__device__ __forceinline__ Sh carve_split(const DevNet& n, unsigned char* sm,
-                                          unsigned char* base) {
+void state_pieces(DevNet& n) {
   size_t os = 0, og = 0;
-  return place_state(n, [&](size_t bytes) {
-    const bool in = os + al16(bytes) <= (size_t)n.sm_state;
-    unsigned char* p = in ? sm + os : base + og;
+  int i = 0;
+  place_state(n, [&](size_t bytes) -> unsigned char* {
+    const bool in = !n.wide || os + al16(bytes) <= (size_t)n.sm_state;
+    n.so[i++] = in ? (int)os : ~(int)og;
     (in ? os : og) += al16(bytes);
-    return p;
+    return nullptr;
   });
 }
 
@@ -1918,7 +1959,7 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
         }
         const double dh = head_of(T.e1[k], s.V1, s.hf) - head_of(T.e2[k], s.V1, s.hf);
         double dq = yk - s.P[k] * dh;
-        if ((n.flags[k] & WDS_F_CHP) && dq > qk) dq = qk / 2.0;
+        if ((T.kf[k] >> 8 & WDS_F_CHP) && dq > qk) dq = qk / 2.0;
         const double q2 = qk - dq;
         s.q[k] = q2;
         sums[0] += fabs(dq);
@@ -1935,6 +1976,16 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
         sums[3] += fabs(en);
       }
     }
+    // the first valve of this thread: its constants, before the reduction's barriers
+    int vk = 0, vpsv = 0;
+    double vhs = 0.0, vkm = 0.0;
+    if (sm && gtid<NT>() < n.npcv) {
+      const int i = gtid<NT>();
+      vk = n.pcv_link[i];
+      vhs = n.pcv_hset[i];
+      vkm = n.pcv_km[i];
+      vpsv = n.pcv_psv[i];
+    }
     block_sum<NT>(sums, 4, s.red);
     const double dqsum = sums[0] + sums[2], qsum = sums[1] + sums[3];
     relerr = qsum > a.hacc ? dqsum / qsum : dqsum;
@@ -1949,14 +2000,20 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
     // ---- batched status machine (hydsolve, solver.py:3126-3179)
     bool vchg = false;
     for (int i = gtid<NT>(); i < n.npcv; i += NT) {
-      const int k = n.pcv_link[i];
+      if (i >= NT) {
+        vk = n.pcv_link[i];
+        vhs = n.pcv_hset[i];
+        vkm = n.pcv_km[i];
+        vpsv = n.pcv_psv[i];
+      }
+      const int k = vk;
       const double h1 = head_of(T.e1[k], s.V1, s.hf), h2 = head_of(T.e2[k], s.V1, s.hf);
-      const double qk = s.q[k], hs = n.pcv_hset[i], ht = n.htol;
+      const double qk = s.q[k], hs = vhs, ht = n.htol;
       const int sk = s.S[k];
-      const double hml = n.pcv_km[i] * (qk * qk);
+      const double hml = vkm * (qk * qk);
       const bool neg = qk < -n.qtol;
       int ns = sk;
-      if (n.pcv_psv[i]) {  // psvstatus (hydstatus.c:302-359 as in dgga/solver.py:1736-1765)
+      if (vpsv) {  // psvstatus (hydstatus.c:302-359 as in dgga/solver.py:1736-1765)
         if (sk == WDS_ACTIVE)
           ns = neg ? WDS_CLOSED : (h2 + hml > hs + ht ? WDS_OPEN : WDS_ACTIVE);
         else if (sk == WDS_OPEN)
@@ -1990,8 +2047,10 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
     bool chg = false;
     if (br_conv || br_per) {
       for (int k = gtid<NT>(); k < n.L; k += NT) {
+        const uint32_t kf = T.kf[k];
         const int st0 = s.S[k];
         int st = (st0 == WDS_XHEAD || st0 == WDS_TEMPCLOSED) ? WDS_OPEN : st0;
+        if (!(kf >> 8 & kStatusLink) && st == st0) continue;  // no rule applies
         const double dh = head_of(T.e1[k], s.V1, s.hf) - head_of(T.e2[k], s.V1, s.hf);
         const double qk = s.q[k];
         if (n.kind[k] == WDS_KIND_CVPIPE) {  // cvstatus
@@ -2125,7 +2184,7 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
     for (int step = 0; step <= a.polish; ++step) {
       bool far = false;
       const bool cand = have && settled;
-      adj_coeffs<NT>(n, th, s, rrow, kerow, cand ? Pf : nullptr, cand ? Ef : nullptr,
+      adj_coeffs<NT>(n, th, T, s, rrow, kerow, cand ? Pf : nullptr, cand ? Ef : nullptr,
                      step == a.polish ? kReuseTerminal : kReuseStep, &far);
       reuse = cand && !gsync_or<NT>(far);
       if (!reuse) {
@@ -2141,8 +2200,11 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
       }
       if (step == a.polish) break;  // terminal factor: keep it
       // residuals (autodiff.py:1032-1050); r_l overwrites Y
+      double yn = gtid<NT>() < n.L ? s.Y[gtid<NT>()] : 0.0;  // the next link's, from L2
       for (int k = gtid<NT>(); k < n.L; k += NT) {
-        const double hl = s.P[k] != 0.0 ? s.Y[k] / s.P[k] : 0.0;
+        const double yk = yn;
+        if (k + NT < n.L) yn = s.Y[k + NT];
+        const double hl = s.P[k] != 0.0 ? yk / s.P[k] : 0.0;
         s.Y[k] = hl - (head_of(T.e1[k], Hs, s.hf) - head_of(T.e2[k], Hs, s.hf));
       }
       bool any_act = false;

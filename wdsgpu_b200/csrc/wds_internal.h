@@ -24,6 +24,19 @@ constexpr int kWideThreads = 1024;
 // 16-byte pieces).
 __host__ __device__ constexpr int top_ld(int nT) { return (nT + 1) & ~1; }
 
+// Bits beside the WDS_F_* flags: the link-status check has a rule for the link
+// (check valve, pump, flow control valve, or a link to a tank); the link has a
+// minor loss.
+constexpr uint32_t kStatusLink = 0x80, kMinorLoss = 0x40;
+
+// A status-machine valve: its link, junctions (n1, n2; the held one and the
+// other), factor slot of the (n1, n2) entry, flow-excess slots (-1: none), head
+// (PRV, PSV) or flow (FCV) setting.
+struct ValveRec {
+  double set, km, sgn;
+  int k, j1, j2, off, x1, x2, jc, jo, fcv, pad;
+};
+
 // Device tables of one network.  Junction vectors are indexed by their
 // elimination index p (0..Nj-1); link ends are "end codes": p >= 0 for a
 // junction, -(f+1) for the f-th fixed-head node.
@@ -103,7 +116,7 @@ struct DevNet {
   // once per CTA (see STabOff)
   const uint4* stab;
   int stab_bytes;
-  int o_spair, o_fpair, o_colptr, o_rowidx, o_levptr, o_rptr, o_rent, o_mode, o_inc_ptr, o_inc_split, o_inc, o_e1, o_e2, o_pptr, o_plink, o_pslot, o_fill, o_dslot;
+  int o_spair, o_fpair, o_colptr, o_rowidx, o_levptr, o_rptr, o_rent, o_mode, o_inc_ptr, o_inc_split, o_inc, o_e1, o_e2, o_pptr, o_plink, o_pslot, o_fill, o_dslot, o_kf, o_vrec;
   // large networks: see factor_rounds
   int o_act, o_term, o_colf, o_colb, o_frnd, o_crnd, o_brnd, o_rptr3;
   // dense top block: levels [L0, nlev) = columns [cT, Nj), nT = Nj - cT
@@ -114,6 +127,8 @@ struct DevNet {
   // large networks: bytes of shared memory that hold the first pieces of the
   // scenario's state
   int sm_state;
+  // offsets of the pieces of a scenario's state (see carve)
+  int so[24];
   // large network: slot-valued tables are 32-bit and stay in global memory
   // with the scenario state (one 256-thread CTA per scenario); otherwise the
   // 16-bit tables are staged into shared memory
@@ -235,6 +250,7 @@ int launch_forward(const DevNet& n, const DevWork& w, const FwdArgs& a, int grou
 int launch_adjoint(const DevNet& n, const DevWork& w, const AdjArgs& a, int groups,
                    void* stream, std::string* err);
 size_t state_smem_bytes(const DevNet& n);
+void state_offsets(DevNet& n);  // n.so, from the sizes, msm and sm_state
 // CTAs of a launch of the adjoint over `rows` rows (-1: a CUDA error in *err)
 int adjoint_grid(const DevNet& n, int groups, int rows, std::string* err);
 

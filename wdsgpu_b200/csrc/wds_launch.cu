@@ -11,6 +11,7 @@
 namespace wds {
 
 size_t state_smem_bytes(const DevNet& n) { return smem_bytes(n); }
+void state_offsets(DevNet& n) { state_pieces(n); }
 
 namespace {
 

@@ -566,6 +566,30 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     jn[p] = jnodes[perm[p]];
     el[p] = net->elev[jn[p]];
   }
+  std::vector<uint16_t> kf(L);
+  for (int k = 0; k < L; ++k) {
+    const int kd = net->link_kind[k];
+    const bool rule = kd == WDS_KIND_CVPIPE || kd == WDS_KIND_PUMP || kd == WDS_KIND_FCV ||
+                      (flags[k] & WDS_F_PUMP_LIVE) || link_tl[k] >= 0;
+    kf[k] = (uint16_t)((kd & 0xff) | ((flags[k] & 0x0f) | (rule ? kStatusLink : 0) |
+                                      (km[k] > 0.0 ? kMinorLoss : 0)) << 8);
+  }
+  std::vector<ValveRec> vrec;
+  for (int v : vord) {
+    ValveRec r{};
+    const int i = v >= 0 ? v : -1 - v;
+    r.fcv = v < 0;
+    if (v >= 0) {
+      r.k = pcv_link[i]; r.j1 = pcv_j1[i]; r.j2 = pcv_j2[i]; r.off = pcv_off[i];
+      r.x1 = pcv_xf[i]; r.x2 = -1; r.jc = pcv_jc[i]; r.jo = pcv_jo[i];
+      r.set = pcv_hset[i]; r.km = pcv_km[i]; r.sgn = pcv_sgn[i];
+    } else {
+      r.k = fcv_link[i]; r.j1 = fcv_j1[i]; r.j2 = fcv_j2[i]; r.off = fcv_off[i];
+      r.x1 = fcv_xf1[i]; r.x2 = fcv_xf2[i]; r.set = fcv_qs[i]; r.km = fcv_km[i];
+    }
+    vrec.push_back(r);
+  }
+  if (vrec.empty()) vrec.push_back(ValveRec{});
   // ---- bounds check of every index the kernels dereference (host side, so
   // that a table error is an error return and never a device fault)
   {
@@ -774,7 +798,7 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     for (auto* v : {&wact, &wterm, &wcf, &wcb})
       if (v->empty()) v->push_back(make_uint4(0, 0, 0, 0));
   };
-  struct TabOff { int sp, fp, cp, ri, lp, rp, re, md, ip, is, in, e1, e2, pp, pl, ps, fl, ds, ac, te, co, cb, rf, rc, rb, r3; };
+  struct TabOff { int sp, fp, cp, ri, lp, rp, re, md, ip, is, in, e1, e2, pp, pl, ps, fl, ds, ac, te, co, cb, rf, rc, rb, r3, kf, vr; };
   auto pack = [&](auto tag, Blob& sb, TabOff& o) {
     using S = decltype(tag);
     constexpr bool W32 = sizeof(S) == 4;
@@ -785,15 +809,14 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
       if (nb) std::memcpy(sb.bytes.data() + off, v.data(), nb);
       return (int)off;
     };
-    // update list of every entry of L, by slot (narrow: begin | count << 16 |
-    // diagonal << 31; wide: begin, count | diagonal << 31)
-    std::vector<uint32_t> sp((size_t)nnzL * (W32 ? 2 : 1), 0);
-    for (auto& t : ftask) {
-      const uint32_t hi = (uint32_t)(t.z - t.y) | ((uint32_t)t.w << 31);
-      if (W32) { sp[2 * (size_t)t.x] = (uint32_t)t.y; sp[2 * (size_t)t.x + 1] = hi; }
-      else sp[t.x] = (uint32_t)t.y | ((uint32_t)(t.z - t.y) << 16) | ((uint32_t)t.w << 31);
+    // update list of every entry of L, by slot: first term | diagonal << 15
+    // (the lists follow one another in slot order)
+    std::vector<uint16_t> sp, fp;
+    if (!W32) {
+      for (auto& f : ftask) sp.push_back((uint16_t)(f.y | f.w << 15));
+      sp.push_back((uint16_t)(fpair.size() / 3));
+      fp.assign(fpair.begin(), fpair.end());
     }
-    std::vector<S> fp(fpair.begin(), fpair.end());
     if (fp.empty()) fp.push_back(0);
     std::vector<S> cp(colptr.begin(), colptr.end());
     // row lists (forward substitution): entries {slot of L_jk, k} of row j at [rptr[j], rptr[j+1])
@@ -810,7 +833,7 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     if (fl.empty()) fl.push_back(0);
     std::vector<S> ds(dsl.size());
     for (size_t i = 0; i < dsl.size(); ++i) ds[i] = dsl[i] < 0 ? (S)~S(0) : (S)dsl[i];
-    o.sp = sadd(sp); o.fp = sadd(fp); o.cp = sadd(cp); o.ri = sadd(s_ri); o.lp = sadd(s_lp);
+    o.vr = sadd(vrec); o.kf = sadd(kf); o.sp = sadd(sp); o.fp = sadd(fp); o.cp = sadd(cp); o.ri = sadd(s_ri); o.lp = sadd(s_lp);
     o.rp = sadd(rp); o.re = sadd(re); o.md = sadd(s_md); o.ip = sadd(s_ip); o.is = sadd(s_is);
     o.in = sadd(s_in); o.e1 = sadd(s_e1); o.e2 = sadd(s_e2); o.pp = sadd(s_pp); o.pl = sadd(s_pl);
     o.ps = sadd(ps); o.fl = sadd(fl); o.ds = sadd(ds);
@@ -821,7 +844,7 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     }
     sb.bytes.resize((sb.bytes.size() + 15) / 16 * 16);
   };
-  const bool fits16 = nnzL < 65535 && (int)fpair.size() / 3 < 65536 &&
+  const bool fits16 = nnzL < 65535 && (int)fpair.size() / 3 < 32768 &&
                       (int)rent.size() < 65536 && (int)fitem.back().z < 65536;
   // per-scenario state of the shared-memory layout (sizes only)
   DevNet dsz{};
@@ -913,6 +936,7 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
   d.wide = wide ? 1 : 0;
   d.fp32 = net->factor_fp32 ? 1 : 0;
   d.stab_bytes = wide ? 0 : (int)stab_bytes.size();  // staged into shared memory (narrow only)
+  d.o_kf = to.kf; d.o_vrec = to.vr;
   d.o_spair = to.sp; d.o_fpair = to.fp; d.o_colptr = to.cp;
   d.o_rowidx = to.ri; d.o_levptr = to.lp; d.o_rptr = to.rp;
   d.o_rent = to.re; d.o_mode = to.md; d.o_inc_ptr = to.ip; d.o_inc_split = to.is;
@@ -966,6 +990,7 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     plan->smem_fwd = best_g ? (size_t)d.stab_bytes + best_g * st : (size_t)d.stab_bytes + st;
     plan->smem_adj = plan->smem_fwd;
   }
+  state_offsets(d);
   if (plan->groups == 0 || (!d.wide && plan->smem_fwd > 227 * 1024)) {
     cudaFree(plan->dtab);
     delete plan;
