@@ -42,14 +42,15 @@ int fail(int code, const std::string& msg) {
 // / entries of L, plain minimum degree -> this: 100 junctions 3 / 289 -> 2 /
 // 294; 542 with 79 TCVs 20 / 1229 -> 5 / 1336; 782 17 / 2327 -> 7 / 2397;
 // 3000 36 / 9922 -> 18 / 10155; 20 000 66 / 63 359 -> 40 / 64 982.  Weights
-// of 1/4 and 1 on the level leave more levels or more entries.
-std::vector<int> min_degree(int n, std::vector<std::vector<int>> adj) {
+// of 1/4 and 1 on the level leave more levels or more entries.  With `plain` the level
+// does not count: the fewest entries.
+std::vector<int> min_degree(int n, std::vector<std::vector<int>> adj, bool plain) {
   std::vector<int> deg(n), lev(n, 0), order;
   order.reserve(n);
   std::vector<char> alive(n, 1);
   // heap of key << 32 | row; an entry whose key is no longer the row's is stale
   std::vector<uint64_t> heap;
-  auto key = [&](int i) { return (uint64_t)(2 * deg[i] + lev[i]) << 32 | (uint32_t)i; };
+  auto key = [&](int i) { return (uint64_t)(2 * deg[i] + (plain ? 0 : lev[i])) << 32 | (uint32_t)i; };
   for (int i = 0; i < n; ++i) {
     deg[i] = (int)adj[i].size();
     heap.push_back(key(i));
@@ -177,7 +178,10 @@ static int groups_for(const WdsPlan* plan, int batch) {
 
 extern "C" const char* wds_last_error(void) { return g_err.c_str(); }
 
-extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out) {
+// wds_plan with the depth-aware order or, `plain`, with the plain minimum-degree
+// order for the small-network layout only (WDS_PLAN_NO_FIT when it does not fit).
+constexpr int WDS_PLAN_NO_FIT = 1;
+static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out, bool plain) {
   using namespace wds;
   if (!net || !out || max_batch <= 0) return fail(WDS_E_ARG, "wds_plan: bad argument");
   *out = nullptr;
@@ -228,7 +232,7 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
       perm[p] = r;
     }
   } else {
-    perm = min_degree(Nj, adj);
+    perm = min_degree(Nj, adj, plain);
   }
   for (int p = 0; p < Nj; ++p) iperm[perm[p]] = p;
   // ---- symbolic factorisation: struct(L_j) = A_{>j,j} U children \ {j}.
@@ -862,6 +866,15 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
     pack(uint16_t{}, sblob, to);
     small_fits = sblob.bytes.size() + state_bytes <= 227 * 1024;
   }
+  if (plain && !small_fits) return WDS_PLAN_NO_FIT;
+  // A network that misses the small layout by little fits it with the order of
+  // the fewest entries (up to 7 % fewer), and runs faster there (1500 junctions,
+  // 1024 scenarios: 4.7 ms against 5.9 on the large layout).
+  if (!small_fits && fits16 && !net->perm && net->layout != WDS_LAYOUT_GLOBAL &&
+      sblob.bytes.size() + state_bytes <= 227 * 1024 * 11 / 10) {
+    const int rc = plan_ordered(net, max_batch, out, true);
+    if (rc != WDS_PLAN_NO_FIT) return rc;
+  }
   const bool wide = !small_fits || net->layout == WDS_LAYOUT_GLOBAL;
   if (wide && net->layout == WDS_LAYOUT_SHARED)
     return fail(WDS_E_UNSUPPORTED, "wds_plan: the network's tables and state exceed shared "
@@ -1026,6 +1039,10 @@ extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out)
   hs.colptr = colptr; hs.rowidx = rowidx;
   *out = plan;
   return WDS_OK;
+}
+
+extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out) {
+  return plan_ordered(net, max_batch, out, false);
 }
 
 extern "C" int wds_plan_stats(const WdsPlan* plan, int64_t* o) {
