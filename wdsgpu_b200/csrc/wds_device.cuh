@@ -616,7 +616,7 @@ __device__ __forceinline__ double amul_node(const DevNet& n, const TB& T, const 
   }
   const int es = s.eslot[p];
   acc = acc + (es >= 0 ? s.em_emh[es] : 0.0) * x[p];
-  for (int c = n.cb_ptr[p]; c < n.cb_ptr[p + 1]; ++c) {
+  for (int c = n.npcv ? n.cb_ptr[p] : 0, ce = n.npcv ? n.cb_ptr[p + 1] : 0; c < ce; ++c) {
     const int i = n.cb_idx[c];
     const double act = S[n.pcv_link[i]] == WDS_ACTIVE ? 1.0 : 0.0;
     acc += x[p] * act * kCBIG;
@@ -1511,7 +1511,7 @@ __device__ void assemble_reduced(const DevNet& n, const TB& T, const Sh& s) {
     for (int e = T.inc_ptr[p]; e < T.inc_ptr[p + 1]; ++e) dg += s.P[inc_link(T, e)];
     const int es = s.eslot[p];
     dg = dg + (es >= 0 ? s.em_emh[es] : 0.0);
-    for (int c = n.cb_ptr[p]; c < n.cb_ptr[p + 1]; ++c) {
+    for (int c = n.npcv ? n.cb_ptr[p] : 0, ce = n.npcv ? n.cb_ptr[p + 1] : 0; c < ce; ++c) {
       const int i = n.cb_idx[c];
       dg += kCBIG * (s.S[n.pcv_link[i]] == WDS_ACTIVE ? 1.0 : 0.0);
     }

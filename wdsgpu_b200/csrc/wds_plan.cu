@@ -143,6 +143,8 @@ wds::DevWork work_at(unsigned char* base, const WorkOff& o, const wds::DevNet& d
 
 struct WdsPlan {
   wds::DevNet dn{};
+  wds::DevNet dn_few{};  // the same for launches of at most `few` groups per CTA
+  int few = 0;
   wds::DevWork dw{};
   wds::HostSym sym;
   void* dtab = nullptr;
@@ -174,6 +176,11 @@ struct WdsPlan {
 static int groups_for(const WdsPlan* plan, int batch) {
   if (plan->tuned) return plan->groups;
   return std::min(plan->groups, std::max(1, (batch + plan->sms - 1) / plan->sms));
+}
+
+// The network's device view for a launch with `groups` groups per CTA.
+static const wds::DevNet& net_for(const WdsPlan* plan, int groups) {
+  return groups <= plan->few ? plan->dn_few : plan->dn;
 }
 
 extern "C" const char* wds_last_error(void) { return g_err.c_str(); }
@@ -1004,6 +1011,18 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
     plan->smem_adj = plan->smem_fwd;
   }
   state_offsets(d);
+  // A launch with fewer groups than the plan's (a batch below its resident
+  // scenarios) has room for the top block's inverse in shared memory.
+  plan->dn_few = d;
+  if (!d.wide && d.nT > 0 && !d.msm) {
+    DevNet& f = plan->dn_few;
+    f.msm = 1;
+    const size_t st = state_smem_bytes(f);
+    while (plan->few < plan->groups - 1 &&
+           (size_t)f.stab_bytes + (plan->few + 1) * st <= 227 * 1024)
+      ++plan->few;
+    state_offsets(f);
+  }
   if (plan->groups == 0 || (!d.wide && plan->smem_fwd > 227 * 1024)) {
     cudaFree(plan->dtab);
     delete plan;
@@ -1122,7 +1141,8 @@ extern "C" int wds_forward(WdsPlan* plan, int32_t batch, const WdsForwardOpts* o
   a.head = head; a.flow = flow; a.emit = emitter; a.status = status; a.iters = iters;
   a.relerr = relerr; a.info = info;
   std::string err;
-  int rc = launch_forward(plan->dn, plan->dw, a, groups_for(plan, batch), stream, &err);
+  const int groups = groups_for(plan, batch);
+  int rc = launch_forward(net_for(plan, groups), plan->dw, a, groups, stream, &err);
   if (rc != WDS_OK) return fail(rc, err);
   plan->have_state = o->polish_steps >= 0;
   plan->state_batch = batch;
@@ -1148,7 +1168,8 @@ extern "C" int wds_adjoint_rhs(WdsPlan* plan, int32_t batch, int32_t rhs_per, in
   a.rhs_per = rhs_per;
   a.v0 = first;
   std::string err;
-  int rc = launch_adjoint(plan->dn, plan->dw, a, groups_for(plan, batch), stream, &err);
+  const int groups = groups_for(plan, batch);
+  int rc = launch_adjoint(net_for(plan, groups), plan->dw, a, groups, stream, &err);
   if (rc != WDS_OK) return fail(rc, err);
   return WDS_OK;
 }
@@ -1179,7 +1200,7 @@ extern "C" int wds_sensitivity(WdsPlan* plan, int32_t rows, int32_t rhs_per, int
   const size_t glob = d.wide && st > (size_t)d.sm_state ? (st + 255) / 256 * 256 : 0;
   const int groups = groups_for(plan, rows);
   if (scr + glob > 0) {
-    const int grid = adjoint_grid(d, groups, rows, &err);
+    const int grid = adjoint_grid(net_for(plan, groups), groups, rows, &err);
     if (grid < 0) return fail(WDS_E_CUDA, err);
     const int slots = grid * groups;
     if (slots > plan->rows_slots) {
@@ -1193,7 +1214,7 @@ extern "C" int wds_sensitivity(WdsPlan* plan, int32_t rows, int32_t rhs_per, int
     if (scr) w.scr = (double*)plan->drows;
     if (glob) w.state = (unsigned char*)plan->drows + (size_t)plan->rows_slots * scr;
   }
-  const int rc = launch_adjoint(d, w, a, groups, stream, &err);
+  const int rc = launch_adjoint(net_for(plan, groups), w, a, groups, stream, &err);
   if (rc != WDS_OK) return fail(rc, err);
   return WDS_OK;
 }
@@ -1284,7 +1305,8 @@ extern "C" int wds_adjoint(WdsPlan* plan, int32_t batch, const double* gH, const
     return fail(WDS_E_STATE, "wds_adjoint: no implicit forward of this batch size to differentiate");
   AdjArgs a{batch, gH, gQ, gE, gd, grh, gke, gr};
   std::string err;
-  int rc = launch_adjoint(plan->dn, plan->dw, a, groups_for(plan, batch), stream, &err);
+  const int groups = groups_for(plan, batch);
+  int rc = launch_adjoint(net_for(plan, groups), plan->dw, a, groups, stream, &err);
   if (rc != WDS_OK) return fail(rc, err);
   return WDS_OK;
 }
@@ -1305,7 +1327,8 @@ extern "C" int wds_adjoint_pumps(WdsPlan* plan, int32_t batch, const double* gH,
   a.gh0 = gh0;
   a.grp = grp;
   std::string err;
-  int rc = launch_adjoint(plan->dn, plan->dw, a, groups_for(plan, batch), stream, &err);
+  const int groups = groups_for(plan, batch);
+  int rc = launch_adjoint(net_for(plan, groups), plan->dw, a, groups, stream, &err);
   if (rc != WDS_OK) return fail(rc, err);
   return WDS_OK;
 }
@@ -1333,7 +1356,8 @@ extern "C" int wds_unrolled_adjoint(WdsPlan* plan, int32_t batch, int32_t K,
   u.ke_stride = ke_stride; u.r = r; u.r_stride = r_stride; u.gH = gH; u.gQ = gQ; u.gE = gE;
   u.gd = gd; u.grh = grh; u.gke = gke; u.gr = gr; u.scr = scratch; u.s0 = status0;
   std::string err;
-  const int rc = launch_unrolled(plan->dn, plan->dw, u, groups_for(plan, batch), stream, &err);
+  const int groups = groups_for(plan, batch);
+  const int rc = launch_unrolled(net_for(plan, groups), plan->dw, u, groups, stream, &err);
   plan->have_state = false;  // the reverse pass reuses the plan's factor workspace
   ++plan->gen;
   if (rc != WDS_OK) return fail(rc, err);
@@ -1427,7 +1451,8 @@ extern "C" int wds_forward_noalloc(const WdsPlan* plan, int32_t batch, const Wds
   a.head = head; a.flow = flow; a.emit = emitter; a.status = status; a.iters = iters;
   a.relerr = relerr; a.info = info;
   std::string err;
-  rc = launch_forward(d, w, a, groups_for(plan, batch), stream, &err);
+  const int groups = groups_for(plan, batch);
+  rc = launch_forward(net_for(plan, groups), w, a, groups, stream, &err);
   if (rc != WDS_OK) return fail(rc, err);
   return WDS_OK;
 }
