@@ -5,23 +5,25 @@
 // through the kernel selectors at the end of this file.
 //
 // A CTA holds `GR` independent scenario groups of 256 threads.  Each group owns
-// one scenario at a time: its link flows and coefficients, the LDL^T factor of
-// the node matrix and the node vectors live in shared memory from the first
-// Newton iteration to the terminal factorisation, so there is no host round
-// trip inside the loop.  The symbolic schedule (update lists, row and column
+// one scenario at a time: its link conductances, the LDL^T factor of the node
+// matrix and the node vectors live in shared memory (its link flows in L2) from
+// the first Newton iteration to the terminal factorisation, so there is no host
+// round trip inside the loop.  A network too large for that runs one scenario
+// per CTA of 1024 threads, its state in shared memory as far as it fits.  The symbolic schedule (update lists, row and column
 // structure, incidence lists) is staged once per CTA into shared memory as
 // 16-bit tables and shared by the groups.  Groups synchronise on their own
 // named barriers, so they advance independently.
 //
 // Per GGA iteration (dgga/solver.py:2922-3179):
-//   link pass    P, Y from the headloss formulas (one thread per link)
+//   link pass    P, Y from the headloss formulas and the link's term of the
+//                right-hand side (one thread per link)
 //   node pass    gather assembly of A (diagonal, pairs) and F in the
-//                reference's scatter order; PRV valve coefficients after the
-//                node coefficients (serial over the few PRVs)
-//   factor       left-looking LDL^T, dependency-driven: a column starts as soon
-//                as the columns it depends on are done (shared-memory counters)
-//   solve        dependency-driven forward/backward substitution + refinement
-//                against the matrix-free operator A x
+//                reference's scatter order; valve coefficients after the node
+//                coefficients (a lane per valve, in valve order)
+//   factor       left-looking LDL^T by elimination-tree level, the top levels
+//                as one dense block inverted on the FP64 tensor cores
+//   solve        forward/backward substitution by level around the top block's
+//                inverse + refinement against the matrix-free operator A x
 //   update       dq = Y - P dh, emitter update, relerr reduction, status
 //                machine (valve status every iteration, link status on the
 //                converged / periodic branches, per-scenario nextcheck)
@@ -893,7 +895,9 @@ __device__ __forceinline__ void top_steps(int nT, int tiles, int w, int lane,
 // tensor-core product: a block costs a warp six of them and 4 FMAs per lane,
 // where four single-column sweeps on 3 x 3 entries per thread cost 48
 // multiplies and FMAs per lane and four barriers of the whole group.  A
-// seventh warp inverts the pivot blocks.  What bounds it is the chain of a
+// seventh warp inverts the pivot blocks (44 columns, alone / three groups per
+// SM: 19.0 / 31.3 k cycles with the single-column sweeps, 11.2 / 16.8 k so).
+// What bounds it is the chain of a
 // block: publish the columns, invert the 4 x 4 block (two reciprocals), read
 // it back, update the next block's tile.  S is read from the factor slots
 // listed in dslot, S^{-1} is written to Mg (row-major, rows of top_ld(nT)
@@ -1426,7 +1430,9 @@ __device__ void assemble_gga(const DevNet& n, const TB& T, const Sh& s, const do
   // valvecoeffs after nodecoeffs, in valve order: a lane of the last warp (the
   // fewest junctions) per valve loads its flow and status and forms its
   // coefficients before the barrier, all valves at once, and the lanes then
-  // take their turns at what depends on the order.
+  // take their turns at what depends on the order (3 valves, three groups per
+  // SM, with the status pass: 9.0 -> 6.0 k cycles an iteration against one
+  // thread that took valve after valve).
   const int nv = n.npcv + n.nfcv, lane = threadIdx.x & 31;
   if (nv == 0) {
     gsync<NT>();
@@ -1749,7 +1755,8 @@ __host__ __device__ __forceinline__ Sh place_state(const DevNet& n, Take&& take)
 // The state at `base` (shared memory on the small-network layout).  The pieces
 // lie at offsets the plan computed, kernel parameters: a piece's address is one
 // addition wherever it is used, not a register held (or spilled) from the
-// start of the scenario on.
+// start of the scenario on (three groups: 372 -> 224 bytes of spill loads; L1
+// beside 220 KB of shared memory does not hold the spills of 768 threads).
 __device__ __forceinline__ Sh carve(const DevNet& n, unsigned char* base) {
   int i = 0;
   return place_state(n, [&](size_t) { return base + n.so[i++]; });
