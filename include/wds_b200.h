@@ -138,8 +138,8 @@ typedef struct WdsNetwork {
 /* WdsNetwork.layout */
 #define WDS_LAYOUT_AUTO   0      /* shared memory when it fits, else global             */
 #define WDS_LAYOUT_SHARED 1      /* 16-bit tables and state in shared memory, or fail   */
-#define WDS_LAYOUT_GLOBAL 2      /* 32-bit tables and state in global memory, one CTA
-                                    per scenario (large networks)                         */
+#define WDS_LAYOUT_GLOBAL 2      /* 32-bit tables in global memory, one CTA per scenario, its
+                                    state in shared memory as far as it fits (large networks) */
 
 /* Options of one forward call. */
 typedef struct WdsForwardOpts {

@@ -130,8 +130,8 @@ struct DevNet {
   // offsets of the pieces of a scenario's state (see carve)
   int so[24];
   // large network: slot-valued tables are 32-bit and stay in global memory
-  // with the scenario state (one 256-thread CTA per scenario); otherwise the
-  // 16-bit tables are staged into shared memory
+  // (one 1024-thread CTA per scenario); otherwise the 16-bit tables are staged
+  // into shared memory
   int wide;
   // factor and substitutions in FP32 (residuals, refinement and the Newton
   // update stay in FP64)
