@@ -1785,6 +1785,7 @@ void state_pieces(DevNet& n) {
     (in ? os : og) += al16(bytes);
     return nullptr;
   });
+  n.gstate = (int)((og + 255) / 256 * 256);
 }
 
 // Bytes of a scenario's state.
@@ -1876,7 +1877,7 @@ __device__ __forceinline__ void cta_rounds(const DevNet& n, const DevWork& w, in
     Sh s;
     if constexpr (TB::kWide)
       s = carve_split(n, smem_raw,
-                      w.state + (size_t)(by_slot ? blk * groups + g : b) * state_bytes);
+                      w.state + (size_t)(by_slot ? blk * groups + g : b) * n.gstate);
     else
       s = carve(n, smem_raw + n.stab_bytes + (size_t)g * state_bytes);
     one(T, s, b);
@@ -2276,7 +2277,7 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
     if (info == 0) {  // store the terminal state for the adjoint
       FT* Wt = reinterpret_cast<FT*>(w.W) + (size_t)b * n.nnzL;
       for (int t = gtid<NT>(); t < n.nnzL; t += NT) Wt[t] = wp<FT>(s)[t];
-      if (n.msm) {
+      if (n.msm && w.M) {
         double* Mt = w.M + (size_t)b * n.nT * top_ld(n.nT);
         for (int t = gtid<NT>(); t < n.nT * top_ld(n.nT); t += NT) Mt[t] = s.Mg[t];
       }

@@ -129,6 +129,7 @@ struct DevNet {
   int sm_state;
   // offsets of the pieces of a scenario's state (see carve)
   int so[24];
+  int gstate;  // bytes of the pieces in the global workspace, per scenario
   // large network: slot-valued tables are 32-bit and stay in global memory
   // (one 1024-thread CTA per scenario); otherwise the 16-bit tables are staged
   // into shared memory

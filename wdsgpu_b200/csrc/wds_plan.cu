@@ -106,10 +106,12 @@ struct Blob {
 // 256-byte aligned.  One function for the plan's own workspace and for the
 // fixed array of wds_forward_noalloc, so the two layouts cannot drift apart.
 struct WorkOff {
-  size_t W, P, dr, emh, hge, dke, act, scr, valid, lk, M, state, pump, dj, bytes;
+  size_t W, P, dr, emh, hge, dke, act, scr, valid, lk, M, state, pump, bytes;
 };
 
-WorkOff work_layout(const wds::DevNet& d, int nscr, size_t B, size_t state_bytes) {
+// Without `keep` there is no room for the terminal top-block inverse where the
+// kernel does not work in it.
+WorkOff work_layout(const wds::DevNet& d, int nscr, size_t B, bool keep) {
   WorkOff o{};
   size_t bytes = 0;
   auto take = [&](size_t n) { size_t off = bytes; bytes += (n + 255) / 256 * 256; return off; };
@@ -117,9 +119,8 @@ WorkOff work_layout(const wds::DevNet& d, int nscr, size_t B, size_t state_bytes
   o.W = take(B * d.nnzL * 8); o.P = take(B * d.L * 8); o.dr = take(B * d.L * 8);
   o.emh = take(B * d.Nj * 8); o.hge = take(B * d.Nj * 8); o.dke = take(B * d.Nj * 8);
   o.act = take(B * pc); o.scr = take(B * (size_t)nscr * d.Nj * 8); o.valid = take(B * 4);
-  o.lk = take(B * 2 * d.L * 8); o.M = take(B * (size_t)std::max(d.nT * wds::top_ld(d.nT), 1) * 8);
-  o.state = take(d.wide ? B * state_bytes : 0); o.pump = take(B * 3 * (size_t)d.npump * 8);
-  o.dj = take(B * d.Nj * 8);
+  o.lk = take(B * 2 * d.L * 8); o.M = take(keep || !d.msm ? B * (size_t)std::max(d.nT * wds::top_ld(d.nT), 1) * 8 : 0);
+  o.state = take(B * (size_t)d.gstate); o.pump = take(B * 3 * (size_t)d.npump * 8);
   o.bytes = bytes;
   return o;
 }
@@ -134,7 +135,7 @@ wds::DevWork work_at(unsigned char* base, const WorkOff& o, const wds::DevNet& d
   w.lk = (double*)(base + o.lk); w.M = (double*)(base + o.M);
   w.state = d.wide ? base + o.state : nullptr;
   w.dpump = (double*)(base + o.pump);
-  w.dj = (double*)(base + o.dj);
+  w.dj = w.dke;  // read until the terminal state, which writes dke, is stored
   w.nscr = nscr;
   return w;
 }
@@ -1043,7 +1044,7 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
   DevWork& w = plan->dw;
   // heads, rp, res, sx, 2p Woodbury columns, 2p+1 per-warp temporaries
   const int nscr = 5 + 4 * std::max(npcv, 1);
-  const WorkOff wo = work_layout(d, nscr, (size_t)max_batch, state_smem_bytes(d));
+  const WorkOff wo = work_layout(d, nscr, (size_t)max_batch, true);
   const size_t bytes = wo.bytes;
   if (cudaMalloc(&plan->dwork, bytes) != cudaSuccess) {
     cudaFree(plan->dtab);
@@ -1195,9 +1196,8 @@ extern "C" int wds_sensitivity(WdsPlan* plan, int32_t rows, int32_t rhs_per, int
   a.by_slot = 1;
   // scratch vectors are read with ACTIVE valves only, the state in global
   // memory only when it exceeds shared memory
-  const size_t st = state_smem_bytes(d);
   const size_t scr = d.npcv > 0 ? ((size_t)w.nscr * d.Nj * 8 + 255) / 256 * 256 : 0;
-  const size_t glob = d.wide && st > (size_t)d.sm_state ? (st + 255) / 256 * 256 : 0;
+  const size_t glob = (size_t)d.gstate;
   const int groups = groups_for(plan, rows);
   if (scr + glob > 0) {
     const int grid = adjoint_grid(net_for(plan, groups), groups, rows, &err);
@@ -1426,9 +1426,10 @@ extern "C" int wds_forward_noalloc(const WdsPlan* plan, int32_t batch, const Wds
     return fail(WDS_E_ARG, "wds_forward_noalloc: null pointer");
   if (o->max_iter <= 0 || !(o->accuracy > 0.0) || o->refine < 0)
     return fail(WDS_E_ARG, "wds_forward_noalloc: bad options");
-  const DevNet& d = plan->dn;
   // the plan's workspace layout, for `batch` scenarios, inside the fixed array
-  const WorkOff wo = work_layout(d, plan->dw.nscr, (size_t)batch, state_smem_bytes(d));
+  const int groups = groups_for(plan, batch);
+  const DevNet& d = net_for(plan, groups);
+  const WorkOff wo = work_layout(d, plan->dw.nscr, (size_t)batch, false);
   if (wo.bytes > (size_t)WDS_NOALLOC_SCRATCH_BYTES) {
     const size_t per = wo.bytes / (size_t)batch;
     return fail(WDS_E_ARG, "wds_forward_noalloc: batch " + std::to_string(batch) + " needs " +
@@ -1440,7 +1441,8 @@ extern "C" int wds_forward_noalloc(const WdsPlan* plan, int32_t batch, const Wds
   void* base = nullptr;
   int rc = scratch_address(&base);
   if (rc != WDS_OK) return rc;
-  const DevWork w = work_at((unsigned char*)base, wo, d, plan->dw.nscr);
+  DevWork w = work_at((unsigned char*)base, wo, d, plan->dw.nscr);
+  if (d.msm) w.M = nullptr;  // no adjoint follows: the inverse is not kept
   FwdArgs a{};
   a.B = batch; a.hacc = o->accuracy; a.max_iter = o->max_iter; a.sm = o->status_machine ? 1 : 0;
   a.refine = o->refine; a.polish = o->polish_steps; a.ke_stride = o->ke_stride;
@@ -1451,8 +1453,7 @@ extern "C" int wds_forward_noalloc(const WdsPlan* plan, int32_t batch, const Wds
   a.head = head; a.flow = flow; a.emit = emitter; a.status = status; a.iters = iters;
   a.relerr = relerr; a.info = info;
   std::string err;
-  const int groups = groups_for(plan, batch);
-  rc = launch_forward(net_for(plan, groups), w, a, groups, stream, &err);
+  rc = launch_forward(d, w, a, groups, stream, &err);
   if (rc != WDS_OK) return fail(rc, err);
   return WDS_OK;
 }
