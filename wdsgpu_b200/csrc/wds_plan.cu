@@ -186,10 +186,11 @@ static const wds::DevNet& net_for(const WdsPlan* plan, int groups) {
 
 extern "C" const char* wds_last_error(void) { return g_err.c_str(); }
 
-// wds_plan with the depth-aware order or, `plain`, with the plain minimum-degree
-// order for the small-network layout only (WDS_PLAN_NO_FIT when it does not fit).
+// wds_plan with the depth-aware order or, `plain` > 0, with the plain
+// minimum-degree order for the small-network layout and at least that many
+// scenario groups per CTA (WDS_PLAN_NO_FIT when they do not fit).
 constexpr int WDS_PLAN_NO_FIT = 1;
-static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out, bool plain) {
+static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out, int plain) {
   using namespace wds;
   if (!net || !out || max_batch <= 0) return fail(WDS_E_ARG, "wds_plan: bad argument");
   *out = nullptr;
@@ -240,7 +241,7 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
       perm[p] = r;
     }
   } else {
-    perm = min_degree(Nj, adj, plain);
+    perm = min_degree(Nj, adj, plain > 0);
   }
   for (int p = 0; p < Nj; ++p) iperm[perm[p]] = p;
   // ---- symbolic factorisation: struct(L_j) = A_{>j,j} U children \ {j}.
@@ -880,7 +881,7 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
   // 1024 scenarios: 4.7 ms against 5.9 on the large layout).
   if (!small_fits && fits16 && !net->perm && net->layout != WDS_LAYOUT_GLOBAL &&
       sblob.bytes.size() + state_bytes <= 227 * 1024 * 11 / 10) {
-    const int rc = plan_ordered(net, max_batch, out, true);
+    const int rc = plan_ordered(net, max_batch, out, 1);
     if (rc != WDS_PLAN_NO_FIT) return rc;
   }
   const bool wide = !small_fits || net->layout == WDS_LAYOUT_GLOBAL;
@@ -994,6 +995,26 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
     };
     int best_g = 4;
     while (best_g > 0 && !fits(0, best_g)) --best_g;
+    // The order of the fewest entries can make room for one group more: taken
+    // for a caller's choice that does not fit otherwise, not by itself (1300
+    // junctions at 1.05 links each, one group depth-aware against two: 148
+    // scenarios 0.69 / 0.97 ms, 1024 3.07 / 3.35; 1100 at 1.2: 0.80 / 0.89,
+    // 3.48 / 3.00).
+    const int want = net->groups_per_cta;
+    if (!plain && !net->perm && want > best_g &&
+        (size_t)d.stab_bytes + want * state_smem_bytes(d) <= 227 * 1024 * 11 / 10) {
+      const int rc = plan_ordered(net, max_batch, out, want);
+      if (rc != WDS_PLAN_NO_FIT) {
+        cudaFree(plan->dtab);
+        delete plan;
+        return rc;
+      }
+    }
+    if (plain > best_g) {
+      cudaFree(plan->dtab);
+      delete plan;
+      return WDS_PLAN_NO_FIT;
+    }
     if (net->groups_per_cta > 0) {  // a tuned choice, if the state fits
       if (!fits(0, net->groups_per_cta)) {
         cudaFree(plan->dtab);
@@ -1062,7 +1083,7 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
 }
 
 extern "C" int wds_plan(const WdsNetwork* net, int32_t max_batch, WdsPlan** out) {
-  return plan_ordered(net, max_batch, out, false);
+  return plan_ordered(net, max_batch, out, 0);
 }
 
 extern "C" int wds_plan_stats(const WdsPlan* plan, int64_t* o) {
