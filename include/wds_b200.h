@@ -305,7 +305,8 @@ int wds_adjoint_rhs(WdsPlan* plan, int32_t batch, int32_t rhs_per, int32_t first
  * (device array [rhs_per]), and gr [rows][L] receives d head / d r.  Any number
  * of rows in one launch (their scratch is by resident scenario, allocated by
  * the first call that needs it and kept by the plan).  As wds_adjoint_rhs with
- * a unit gH row and zero gQ, gE. */
+ * a unit gH row and zero gQ, gE.  The row of an index that is not a junction's
+ * is zero (a fixed head depends on no resistance). */
 int wds_sensitivity(WdsPlan* plan, int32_t rows, int32_t rhs_per, int32_t first,
                     const int32_t* nodes, double* gr, void* stream);
 

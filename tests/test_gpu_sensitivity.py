@@ -72,3 +72,20 @@ def test_sensitivity_at_call_pump_speeds(cuda):
     S0 = sensitivity_matrix(s, inp["demand"], inp["res_head"], None, inp["sensors"], wrt="r",
                             accuracy=1e-7)
     assert np.abs(S - S0).max() > 1e-6 * np.abs(R).max()     # the speeds matter
+
+
+def test_negative_sensor_indices_count_from_the_last_node(cuda):
+    """Node i - N is node i: the same rows, bit for bit."""
+    from wdsgpu_b200 import synth
+    from wdsgpu_b200.sensitivity import sensitivity_matrix
+    from wdsgpu_b200.solver import GGASolver
+    net = synth.looped_network(3, 100, 1, 120, n_emitters=5)
+    d, _ = synth.config2_scenarios(net, 2, seed=4)
+    rh = np.broadcast_to(np.nan_to_num(net.fixed_head_ft_at(0)), d.shape).copy()
+    sens = synth.sensor_nodes(net, 6, seed=2)
+    s = GGASolver(net, device=cuda, dense_status_machine=True)
+    S = sensitivity_matrix(s, d, rh, None, sens, wrt="r", accuracy=1e-8)
+    mixed = np.where(np.arange(sens.size) % 2, sens, np.asarray(sens) - net.N)
+    Sn = sensitivity_matrix(s, d, rh, None, mixed, wrt="r", accuracy=1e-8)
+    assert np.abs(S).max(1).min() > 0.0
+    assert np.array_equal(S, Sn)
