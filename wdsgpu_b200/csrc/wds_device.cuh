@@ -253,8 +253,8 @@ __device__ void block_maxmin(double& mx, double& mn, double* red) {
 }
 
 // ---------------------------------------------------------------- formulas
-// 1 / x for a positive normal x to about one unit in the last place: the
-// hardware's 23-bit approximation and two Newton steps (48 cycles of latency
+// 1 / x for a normal x in (0, 2^1021) to about one unit in the last place (0 and
+// infinity give NaN): the hardware's 23-bit approximation and two Newton steps (48 cycles of latency
 // against 77 of the correctly rounded __drcp_rn, measured on dependent
 // chains).
 __device__ __forceinline__ double recip(double x) {
@@ -360,24 +360,38 @@ __device__ __forceinline__ void valve_open(const DevNet& n, double q, double km,
   }
 }
 
+// pipe_coef where the gradient hg (the friction part h0 of it) or the head loss
+// leaves the range of a double: the plain divisions.  An infinite gradient gives
+// P = 0 and Y = NaN, so the scenario does not converge and no pivot fails.
+__device__ __noinline__ double2 pipe_over(double h0, double hg, double ex, double qa, double sgn,
+                                          double km) {
+  const double hl = h0 * qa / ex;
+  return make_double2(1.0 / hg, (km > 0.0 ? hl + km * qa * qa : hl) * sgn / hg);
+}
+
 // pipecoeff, Hazen-Williams / Chezy-Manning (dgga/solver.py:2176-2201)
 __device__ __forceinline__ void pipe_coef(const DevNet& n, double q, double r, double km,
                                           double& P, double& Y) {
   const double sgn = q < 0.0 ? -1.0 : 1.0;
   const double qa = q * sgn;
-  double hg = n.hexp * r * pow_pos(fmax(qa, 1e-30), n.hexp - 1.0);
-  const bool lin = hg < n.rqtol;
-  if (lin) hg = n.rqtol;
-  const double ex = lin ? 1.0 : n.hexp;  // hl = hg qa / ex
-  if (km > 0.0) {
-    const double hl = quotient(hg * qa, ex, lin ? 1.0 : n.rhexp) + km * qa * qa;
-    hg = hg + 2.0 * km * qa;
-    P = recip(hg);
-    Y = quotient(hl, hg, P) * sgn;
-  } else {
-    P = recip(hg);
-    Y = quotient(q, ex, lin ? 1.0 : n.rhexp);
+  double h0 = n.hexp * r * pow_pos(fmax(qa, 1e-30), n.hexp - 1.0);
+  const bool lin = h0 < n.rqtol;
+  if (lin) h0 = n.rqtol;
+  const double ex = lin ? 1.0 : n.hexp, rex = lin ? 1.0 : n.rhexp;  // hl = h0 qa / ex
+  const double hg = km > 0.0 ? h0 + 2.0 * km * qa : h0;
+  // exponents of hg and hg qa at 1021 and above (infinities and NaN among them)
+  if ((unsigned)(__double2hiint(hg) & 0x7fffffff) +
+          (unsigned)max(__double2hiint(qa) & 0x7fffffff, 0x3ff00000) >= 0xbfb00000u) {
+    const double2 c = pipe_over(h0, hg, ex, qa, sgn, km);
+    P = c.x;
+    Y = c.y;
+    return;
   }
+  P = recip(hg);
+  if (km > 0.0)
+    Y = quotient(quotient(h0 * qa, ex, rex) + km * qa * qa, hg, P) * sgn;
+  else
+    Y = quotient(q, ex, rex);
 }
 
 // Pump parameters of one scenario: rows of [L] values read at pump links
