@@ -191,3 +191,30 @@ def test_clamp_branch_in_multi_and_eps_routes(cuda):
     g_dem = eo.backward(runs, gH, gQ, gE, gT, P=T)[0]
     G = D.grad.cpu().numpy()
     assert np.abs(G - g_dem).max() <= 1e-7 * np.abs(g_dem).max()
+
+
+def test_refused_speed_leaves_the_kept_state(cuda):
+    """A speed off the link settings of a non-pump link is refused before
+    anything is launched: the plan's kept state, and so a second backward of
+    an earlier forward, is untouched."""
+    from wdsgpu_b200.autodiff import implicit_solve
+    from wdsgpu_b200.solver import GGASolver
+    net, inp, _ = load("pump_ref")
+    s = GGASolver(net, device=cuda, dense_status_machine=True)
+    B = inp["demand"].shape[0]
+    D = torch.tensor(inp["demand"], device=cuda).requires_grad_(True)
+    RH = torch.tensor(np.nan_to_num(inp["res_head"]), device=cuda)
+    speed = torch.tensor(inp["speed"], device=cuda)
+    loss = (implicit_solve(s, D, RH, accuracy=1e-7, speed=speed)[0] ** 2).sum()
+    g1, = torch.autograd.grad(loss, D, retain_graph=True)
+    plan, gen = s.plan(B), s.plan(B).generation()
+    off = int(np.flatnonzero(~np.isin(np.arange(net.L), net.pump_link))[0])
+    bad = speed.clone()
+    bad[..., off] += 0.5
+    for call in (lambda: implicit_solve(s, D, RH, accuracy=1e-7, speed=bad),
+                 lambda: implicit_solve(s, D, RH, accuracy=1e-30, max_iter=1, speed=bad)):
+        with pytest.raises(NotImplementedError, match="off pump links"):
+            call()
+    assert s.plan(B) is plan and plan.generation() == gen
+    g2, = torch.autograd.grad(loss, D)
+    assert torch.equal(g1, g2)

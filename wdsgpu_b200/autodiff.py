@@ -193,15 +193,11 @@ class ImplicitGGASolveSM100(torch.autograd.Function):
         if ke_t.shape[0] == 1 and B > 1:
             ke_t = ke_t.contiguous()
         th_in = (speed, pump_h0, pump_r)
-        later = []
-        pumps = s.pump_rows(B, *th_in, later=later)
+        pumps = s.pump_rows(B, *th_in)
         o = s.run(d, rh, ke_t, r_t, B, int(max_iter), float(accuracy), sm, int(polish_steps),
                   pumps=pumps)
         info = o["info"]
-        host_info = info.cpu().numpy()   # the host's one wait when every scenario converged
-        for check in later:
-            check()
-        if host_info.any():
+        if info.cpu().numpy().any():   # the host's one wait when every scenario converged
             from .solver import _check_info_flags
             _check_info_flags(s, info)
             bad = torch.nonzero(info != 0).flatten().tolist()

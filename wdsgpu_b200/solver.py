@@ -626,13 +626,10 @@ class GGASolver:
             return 0.0
         return 1e-5
 
-    def pump_rows(self, B, speed=None, pump_h0=None, pump_r=None, later=None):
+    def pump_rows(self, B, speed=None, pump_h0=None, pump_r=None):
         """Pump parameters of a call as FP64 device rows: (speed, h0, r), each
         None or [1, L] / [B, L] with one common row count (an [L] row next to
-        [B, L] rows is expanded).  Values off pump links are not read.  With a
-        list `later`, the comparison of speed with the link settings off pump
-        links is appended to it as a function to call once the host waits for
-        the call's results anyway."""
+        [B, L] rows is expanded).  Values off pump links are not read."""
         vals = [speed, pump_h0, pump_r]
         if all(v is None for v in vals):
             return None
@@ -653,32 +650,25 @@ class GGASolver:
                 # the reference's speed is the whole link-setting vector
                 # (LinkSetting, dgga/autodiff.py:99-120); off pump links it
                 # would set valve settings, which this route does not take
-                check = self._speed_check(t)
-                if later is None:
-                    check()
-                else:
-                    later.append(check)
+                self._check_speed(t)
             out.append(t)
         rows = max(t.shape[0] for t in out if t is not None)
         return tuple(None if t is None else t.expand(rows, L).contiguous() for t in out)
 
-    def _speed_check(self, t):
-        """Compares speed rows [., L] with the link settings off pump links, on
-        the device; the returned function reads the result and raises."""
+    def _check_speed(self, t):
+        """Refuses speed rows [., L] that differ from the link settings off pump
+        links.  The comparison runs on the device; the host waits for it, so
+        that a refused call launches nothing and no plan's kept state is lost."""
         if self._off_pumps is None:
             self._off_pumps = (torch.as_tensor(self._lt != PUMP, device=self.device),
                                torch.as_tensor(self.init_setting, device=self.device))
         off, ref = self._off_pumps
-        hit = ((t != ref) & off).any()
-
-        def check():
-            if bool(hit):
-                bad = torch.nonzero(((t != ref) & off).any(0)).flatten()
-                raise NotImplementedError(
-                    "speed differs from the network's link settings off pump links "
-                    "(links %s): valve settings are not parameters of this route"
-                    % bad[:8].tolist())
-        return check
+        hit = (t != ref) & off
+        if bool(hit.any()):
+            raise NotImplementedError(
+                "speed differs from the network's link settings off pump links "
+                "(links %s): valve settings are not parameters of this route"
+                % torch.nonzero(hit.any(0)).flatten()[:8].tolist())
 
     def run(self, d, rh, ke, r, B, max_iter, hacc, status_machine, polish_steps,
             refine=None, plan=None, q0=None, e0=None, pumps=None, refine_band=None,
