@@ -58,7 +58,8 @@ constexpr double kReuseFlow = 1e-6;
 struct Sh {
   double *q, *P, *Y, *W, *V0, *V1, *V2, *hf, *xf, *red, *small;
   float* Wf;                      // the factor when it is kept in FP32 (W is then null)
-  // per emitter slot: flow, coefficient, 1/hgrad, head loss, elevation
+  // per emitter slot: flow, coefficient, 1/hgrad, head loss, elevation (the
+  // last two outside the state with n.ems = 0, see em_hloss)
   double *em_e, *em_ke, *em_emh, *em_hl, *em_el;
   int16_t* eslot;                 // [Nj] emitter slot of a junction or -1
   double* tb;                     // scratch of the top-block inversion (V2's storage)
@@ -92,11 +93,11 @@ struct TabT {
   const uint8_t* mbwd;
   const uint16_t* inc_ptr;    // [Nj+1]
   const uint16_t* inc_split;  // [Nj]
-  const uint32_t* inc;        // link | PRV << 16 | other fixed << 17 | fixed index << 18
+  const uint16_t* inc;        // links at the junctions
   const int16_t* e1;          // [L] end codes
   const int16_t* e2;
   const uint16_t* pptr;       // [npairs+1]
-  const uint16_t* plink;      // link | PRV << 15
+  const uint16_t* plink;      // links of the pairs
   const Slot* pslot;          // [npairs]
   const Slot* fill;           // [nfill]
   // large networks (kWide): factor entries, their terms, column records of the
@@ -154,7 +155,7 @@ __device__ TB tab_view(const DevNet& n, const unsigned char* b) {
   t.mbwd = t.mfwd + n.nlev;
   t.inc_ptr = (const uint16_t*)(b + n.o_inc_ptr);
   t.inc_split = (const uint16_t*)(b + n.o_inc_split);
-  t.inc = (const uint32_t*)(b + n.o_inc);
+  t.inc = (const uint16_t*)(b + n.o_inc);
   t.e1 = (const int16_t*)(b + n.o_e1);
   t.e2 = (const int16_t*)(b + n.o_e2);
   t.pptr = (const uint16_t*)(b + n.o_pptr);
@@ -175,9 +176,11 @@ __device__ TB tab_view(const DevNet& n, const unsigned char* b) {
   return t;
 }
 
-// link index of an incidence entry (the upper bits carry flags)
-template <class TB>
-__device__ __forceinline__ int inc_link(const TB& T, int e) { return (int)(T.inc[e] & 0xffffu); }
+// a link (kf: its entry of that table) whose coefficients the valve pass forms
+__device__ __forceinline__ bool valve_link(uint32_t kf) {
+  const int kd = (int)(kf & 0xff);
+  return kd == WDS_KIND_PRV || kd == WDS_KIND_PSV || kd == WDS_KIND_FCV;
+}
 
 __device__ __forceinline__ double head_of(int c, const double* x, const double* hf) {
   return c >= 0 ? x[c] : hf[-c - 1];
@@ -623,11 +626,11 @@ __device__ __forceinline__ double amul_node(const DevNet& n, const TB& T, const 
   double acc = 0.0;
   const int a = T.inc_ptr[p], m = T.inc_split[p], z = T.inc_ptr[p + 1];
   for (int e = a; e < m; ++e) {
-    const int k = inc_link(T, e);
+    const int k = T.inc[e];
     acc += P[k] * (junc_of(T.e1[k], x) - junc_of(T.e2[k], x));
   }
   for (int e = m; e < z; ++e) {
-    const int k = inc_link(T, e);
+    const int k = T.inc[e];
     acc += -(P[k] * (junc_of(T.e1[k], x) - junc_of(T.e2[k], x)));
   }
   const int es = s.eslot[p];
@@ -1353,6 +1356,25 @@ __device__ void dense_solve(double* C, double* y, int m) {
 }
 
 // ---------------------------------------------------------------- assembly
+// Head loss of emitter slot es and elevation of its junction p: in the state, or
+// (n.ems = 0, where it has no room for them) the losses in hl, the scenario's row
+// of hge that the terminal state takes over, the elevations in the network's
+// table.  Shared and global loads by a branch that every thread takes alike: one
+// pointer for both makes every load of the two generic (782 junctions, 16 384
+// scenarios: 41.4 ms against 40.9).
+__device__ __forceinline__ double em_hloss(const DevNet& n, const Sh& s, const double* hl, int es) {
+  double v;
+  if (n.ems) v = s.em_hl[es];
+  else asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(hl + es));
+  return v;
+}
+__device__ __forceinline__ double em_elev(const DevNet& n, const Sh& s, int p, int es) {
+  double v;
+  if (n.ems) v = s.em_el[es];
+  else asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(n.el + p));
+  return v;
+}
+
 // Headloss stage of a GGA iteration (dgga/solver.py:2923-2956): P and Y of every
 // link, and 1/hgrad and head loss of every emitter.  What a link adds to the
 // right-hand side at its ends is formed here too, once, into the solves'
@@ -1364,7 +1386,7 @@ __device__ void dense_solve(double* C, double* y, int m) {
 // junctions, three groups per SM: 18.5 -> 4.7 k cycles an iteration).
 template <int NT, class TB>
 __device__ void link_pass(const DevNet& n, const PumpTh& th, const TB& T, const Sh& s,
-                          const double* rrow) {
+                          const double* rrow, double* hrow) {
   const int tid = gtid<NT>();
   double* Z = s.V2;
   // the next link's flow and resistance, in L2, are loaded while this link's
@@ -1387,13 +1409,13 @@ __device__ void link_pass(const DevNet& n, const PumpTh& th, const TB& T, const 
     double z = Y - qk;
     if (c2 < 0 && c1 >= 0) z += P * s.hf[-c2 - 1];
     if (c1 < 0 && c2 >= 0) z -= P * s.hf[-c1 - 1];
-    const int kd = (int)(kf & 0xff);
-    Z[k] = kd == WDS_KIND_PRV || kd == WDS_KIND_PSV || kd == WDS_KIND_FCV ? 0.0 : z;
+    Z[k] = valve_link(kf) ? 0.0 : z;
   }
   for (int es = tid; es < s.flag[2]; es += NT) {
     double hl, hg;
     emitter_hl(n, s.em_e[es], s.em_ke[es], hl, hg);
-    s.em_hl[es] = hl;
+    if (n.ems) s.em_hl[es] = hl;
+    else hrow[es] = hl;
     s.em_emh[es] = 1.0 / hg;
   }
 }
@@ -1402,7 +1424,8 @@ __device__ void link_pass(const DevNet& n, const PumpTh& th, const TB& T, const 
 // emittercoeffs -> nodecoeffs, solver.py:2958-3007) from the link pass, into W
 // (pattern of L) and F = V0; Xflow saved for the junctions whose valves read it.
 template <int NT, class FT, class TB>
-__device__ void assemble_gga(const DevNet& n, const TB& T, const Sh& s, const double* dj) {
+__device__ void assemble_gga(const DevNet& n, const TB& T, const Sh& s, const double* dj,
+                             const double* hrow) {
   const int tid = gtid<NT>();
   const double* Z = s.V2;
   for (int p = tid; p < n.Nj; p += NT) {
@@ -1411,14 +1434,14 @@ __device__ void assemble_gga(const DevNet& n, const TB& T, const Sh& s, const do
     const int es = s.eslot[p];
     double dg = 0.0, F = 0.0;
     for (int e = a; e < z; ++e) {
-      const int k = inc_link(T, e);
+      const int k = T.inc[e];
       dg += s.P[k];
       F += e < m ? Z[k] : -Z[k];
     }
     if (es >= 0) {
       const double emh = s.em_emh[es];
       dg = dg + emh;
-      F = F + (s.em_hl[es] + s.em_el[es]) * emh - s.em_e[es];
+      F = F + (em_hloss(n, s, hrow, es) + em_elev(n, s, p, es)) * emh - s.em_e[es];
     }
     wp<FT>(s)[T.colptr[p]] = (FT)dg;
     s.V0[p] = F - dem;
@@ -1427,8 +1450,8 @@ __device__ void assemble_gga(const DevNet& n, const TB& T, const Sh& s, const do
     const int p = n.xf_node[i], m = T.inc_split[p], z = T.inc_ptr[p + 1];
     double xf = 0.0;
     for (int e = T.inc_ptr[p]; e < z; ++e) {
-      const uint32_t ie = T.inc[e];
-      const double q = ie & (1u << 16) ? 0.0 : s.q[ie & 0xffff];
+      const int k = T.inc[e];
+      const double q = valve_link(T.kf[k]) ? 0.0 : s.q[k];
       xf += e < m ? -q : q;
     }
     const int es = s.eslot[p];
@@ -1437,7 +1460,7 @@ __device__ void assemble_gga(const DevNet& n, const TB& T, const Sh& s, const do
   }
   for (int t = tid; t < n.npairs; t += NT) {
     double v = 0.0;
-    for (int e = T.pptr[t]; e < T.pptr[t + 1]; ++e) v += -s.P[T.plink[e] & 0x7fff];
+    for (int e = T.pptr[t]; e < T.pptr[t + 1]; ++e) v += -s.P[T.plink[e]];
     wp<FT>(s)[T.pslot[t]] = (FT)v;
   }
   for (int t = tid; t < n.nfill; t += NT) wp<FT>(s)[T.fill[t]] = FT(0);
@@ -1528,7 +1551,7 @@ __device__ void assemble_reduced(const DevNet& n, const TB& T, const Sh& s) {
   const int tid = gtid<NT>();
   for (int p = tid; p < n.Nj; p += NT) {
     double dg = 0.0;
-    for (int e = T.inc_ptr[p]; e < T.inc_ptr[p + 1]; ++e) dg += s.P[inc_link(T, e)];
+    for (int e = T.inc_ptr[p]; e < T.inc_ptr[p + 1]; ++e) dg += s.P[T.inc[e]];
     const int es = s.eslot[p];
     dg = dg + (es >= 0 ? s.em_emh[es] : 0.0);
     for (int c = n.npcv ? n.cb_ptr[p] : 0, ce = n.npcv ? n.cb_ptr[p + 1] : 0; c < ce; ++c) {
@@ -1539,7 +1562,7 @@ __device__ void assemble_reduced(const DevNet& n, const TB& T, const Sh& s) {
   }
   for (int t = tid; t < n.npairs; t += NT) {
     double v = 0.0;
-    for (int e = T.pptr[t]; e < T.pptr[t + 1]; ++e) v += -s.P[T.plink[e] & 0x7fff];
+    for (int e = T.pptr[t]; e < T.pptr[t + 1]; ++e) v += -s.P[T.plink[e]];
     wp<FT>(s)[T.pslot[t]] = (FT)v;
   }
   for (int t = tid; t < n.nfill; t += NT) wp<FT>(s)[T.fill[t]] = FT(0);
@@ -1554,8 +1577,7 @@ __device__ void assemble_reduced(const DevNet& n, const TB& T, const Sh& s) {
 // coefficients are formed.
 template <int NT, class TB>
 __device__ void adj_coeffs(const DevNet& n, const PumpTh& th, const TB& T, const Sh& s,
-                           const double* rrow,
-                           const double* kerow, const double* Pf = nullptr,
+                           const double* rrow, double* hrow, const double* Pf = nullptr,
                            const double* Ef = nullptr, double tol = 0.0,
                            bool* far = nullptr) {
   const int tid = gtid<NT>();
@@ -1583,7 +1605,8 @@ __device__ void adj_coeffs(const DevNet& n, const PumpTh& th, const TB& T, const
     double hl, hg;
     emitter_hl(n, s.em_e[es], s.em_ke[es], hl, hg);
     const double emh = 1.0 / hg;
-    s.em_hl[es] = hl;
+    if (n.ems) s.em_hl[es] = hl;
+    else hrow[es] = hl;
     s.em_emh[es] = emh;
     if (Ef) fr = fr || !(fabs(emh - e0) <= tol * fabs(e0));
   }
@@ -1727,7 +1750,11 @@ __host__ __device__ __forceinline__ size_t al16(size_t x) { return (x + 15) / 16
 // then the vector the substitutions run in, the solution, the factor, the
 // conductances and the rest.  take(bytes) places a piece and returns its
 // address (null when only sizes are wanted).
-template <class Take>
+// On the small layout V1 follows V2, and with n.join V2 is a node vector that
+// runs on into V1 where the link pass or the top block's inversion needs more:
+// V1, the heads, is set by the solve after both (a network of more links than
+// junctions then needs no more room for the link pass).
+template <bool kWide, class Take>
 __host__ __device__ __forceinline__ Sh place_state(const DevNet& n, Take&& take) {
   Sh s;
   s.q = nullptr;  // link flows and Y live in the global workspace (set by the kernel)
@@ -1742,16 +1769,19 @@ __host__ __device__ __forceinline__ Sh place_state(const DevNet& n, Take&& take)
   s.em_e = (double*)take(8ull * n.emcap);
   s.em_ke = (double*)take(8ull * n.emcap);
   s.em_emh = (double*)take(8ull * n.emcap);
-  s.em_hl = (double*)take(8ull * n.emcap);
-  s.em_el = (double*)take(8ull * n.emcap);
+  s.em_hl = (double*)take(n.ems ? 8ull * n.emcap : 0);
+  s.em_el = (double*)take(n.ems ? 8ull * n.emcap : 0);
   // the solves' temporary; idle while the matrix is factored, so the top
   // block's inversion works there
-  s.V2 = (double*)take(8ull * v2_len(n));
+  const size_t jv = 8ull * n.Nj, lv = 8ull * v2_len(n);
+  const bool join = !kWide && n.join;
+  s.V2 = (double*)take(join ? jv : lv);
   s.tb = s.V2;
+  if (!kWide) s.V1 = (double*)take(join && lv > al16(jv) + jv ? lv - al16(jv) : jv);
   // the top block's inverse, where it fits (else the kernel points it to the
   // scenario's slice of the global workspace)
   s.Mg = n.msm ? (double*)take(8ull * n.nT * top_ld(n.nT)) : nullptr;
-  s.V1 = (double*)take(8ull * n.Nj);
+  if (kWide) s.V1 = (double*)take(jv);
   if (n.fp32) {
     s.Wf = (float*)take(4ull * n.nnzL);
     s.W = nullptr;
@@ -1773,7 +1803,7 @@ __host__ __device__ __forceinline__ Sh place_state(const DevNet& n, Take&& take)
 // beside 220 KB of shared memory does not hold the spills of 768 threads).
 __device__ __forceinline__ Sh carve(const DevNet& n, unsigned char* base) {
   int i = 0;
-  return place_state(n, [&](size_t) { return base + n.so[i++]; });
+  return place_state<false>(n, [&](size_t) { return base + n.so[i++]; });
 }
 
 // The state of the large-network layout: a piece in shared memory at `sm`, or
@@ -1781,7 +1811,7 @@ __device__ __forceinline__ Sh carve(const DevNet& n, unsigned char* base) {
 __device__ __forceinline__ Sh carve_split(const DevNet& n, unsigned char* sm,
                                           unsigned char* base) {
   int i = 0;
-  return place_state(n, [&](size_t) {
+  return place_state<true>(n, [&](size_t) {
     const int o = n.so[i++];
     return o >= 0 ? sm + o : base + ~o;
   });
@@ -1793,22 +1823,26 @@ __device__ __forceinline__ Sh carve_split(const DevNet& n, unsigned char* sm,
 void state_pieces(DevNet& n) {
   size_t os = 0, og = 0;
   int i = 0;
-  place_state(n, [&](size_t bytes) -> unsigned char* {
+  auto take = [&](size_t bytes) -> unsigned char* {
     const bool in = !n.wide || os + al16(bytes) <= (size_t)n.sm_state;
     n.so[i++] = in ? (int)os : ~(int)og;
     (in ? os : og) += al16(bytes);
     return nullptr;
-  });
+  };
+  if (n.wide) place_state<true>(n, take);
+  else place_state<false>(n, take);
   n.gstate = (int)((og + 255) / 256 * 256);
 }
 
 // Bytes of a scenario's state.
 size_t smem_bytes(const DevNet& n) {
   size_t o = 0;
-  place_state(n, [&](size_t bytes) -> unsigned char* {
+  auto take = [&](size_t bytes) -> unsigned char* {
     o += al16(bytes);
     return nullptr;
-  });
+  };
+  if (n.wide) place_state<true>(n, take);
+  else place_state<false>(n, take);
   return o;
 }
 
@@ -1841,7 +1875,7 @@ __device__ bool build_emitters(const DevNet& n, const Sh& s, const double* val, 
         s.em_ke[slot] = v;
         s.em_e[slot] = 1.0;
         s.em_emh[slot] = 0.0;
-        s.em_el[slot] = n.el[p];
+        if (n.ems) s.em_el[slot] = n.el[p];
       } else {
         s.eslot[p] = -1;
         if (em) over = true;
@@ -1950,9 +1984,9 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
         r[n.L + p] = s.eslot[p] >= 0 ? s.em_e[s.eslot[p]] : 0.0;
     }
     // ---- headloss coefficients, assembly
-    link_pass<NT>(n, th, T, s, rrow);
+    link_pass<NT>(n, th, T, s, rrow, w.hge + (size_t)b * n.Nj);
     gsync<NT>();
-    assemble_gga<NT, FT>(n, T, s, dj);
+    assemble_gga<NT, FT>(n, T, s, dj, w.hge + (size_t)b * n.Nj);
     ran = true;
     if (!factor<NT, FT>(n, T, s)) {
       info = WDS_INFO_NOT_PD;
@@ -1991,7 +2025,8 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
     for (int p = gtid<NT>(); p < n.Nj; p += NT) {
       const int es = s.eslot[p];
       if (es >= 0) {
-        const double dqe = (s.em_hl[es] - (s.V1[p] - s.em_el[es])) * s.em_emh[es];
+        const double hl = em_hloss(n, s, w.hge + (size_t)b * n.Nj, es);
+        const double dqe = (hl - (s.V1[p] - em_elev(n, s, p, es))) * s.em_emh[es];
         const double en = s.em_e[es] - dqe;
         s.em_e[es] = en;
         sums[2] += fabs(dqe);
@@ -2152,8 +2187,8 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
     for (int p = gtid<NT>(); p < n.Nj; p += NT) {
       double dg = 0.0;
       for (int e = T.inc_ptr[p]; e < T.inc_ptr[p + 1]; ++e) {
-        const uint32_t ie = T.inc[e];
-        dg += ie & (1u << 16) ? 0.0 : s.P[ie & 0xffff];
+        const int k = T.inc[e];
+        dg += valve_link(T.kf[k]) ? 0.0 : s.P[k];
       }
       if (s.eslot[p] >= 0) dg = dg + s.em_emh[s.eslot[p]];
       s.V0[p] = dg;
@@ -2206,8 +2241,8 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
     for (int step = 0; step <= a.polish; ++step) {
       bool far = false;
       const bool cand = have && settled;
-      adj_coeffs<NT>(n, th, T, s, rrow, kerow, cand ? Pf : nullptr, cand ? Ef : nullptr,
-                     step == a.polish ? kReuseTerminal : kReuseStep, &far);
+      adj_coeffs<NT>(n, th, T, s, rrow, w.hge + (size_t)b * n.Nj, cand ? Pf : nullptr,
+                     cand ? Ef : nullptr, step == a.polish ? kReuseTerminal : kReuseStep, &far);
       reuse = cand && !gsync_or<NT>(far);
       if (!reuse) {
         assemble_reduced<NT, FT>(n, T, s);
@@ -2240,19 +2275,20 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
         const int a0 = T.inc_ptr[p], m = T.inc_split[p], z = T.inc_ptr[p + 1];
         double mm = 0.0, bt = 0.0;
         for (int e = m; e < z; ++e) {
-          const int k = inc_link(T, e);
+          const int k = T.inc[e];
           mm += s.q[k];
           bt += s.P[k] * s.Y[k];
         }
         for (int e = a0; e < m; ++e) {
-          const int k = inc_link(T, e);
+          const int k = T.inc[e];
           mm += -s.q[k];
           bt += -(s.P[k] * s.Y[k]);
         }
         const int es = s.eslot[p];
         double re = 0.0, emh = 0.0;
         if (es >= 0) {
-          re = s.em_hl[es] - (Hs[p] - s.em_el[es]);
+          const double hl = em_hloss(n, s, w.hge + (size_t)b * n.Nj, es);
+          re = hl - (Hs[p] - em_elev(n, s, p, es));
           mm = mm - s.em_e[es];
           emh = s.em_emh[es];
         }
@@ -2280,7 +2316,8 @@ __device__ __forceinline__ void forward_one(const DevNet& n, const DevWork& w, c
       for (int p = gtid<NT>(); p < n.Nj; p += NT) {
         const int es = s.eslot[p];
         if (es >= 0) {
-          const double re = s.em_hl[es] - (Hs[p] - s.em_el[es]);
+          const double hl = em_hloss(n, s, w.hge + (size_t)b * n.Nj, es);
+          const double re = hl - (Hs[p] - em_elev(n, s, p, es));
           s.em_e[es] = s.em_e[es] + (s.V1[p] - re) * s.em_emh[es];
         }
         Hs[p] = Hs[p] + s.V1[p];
@@ -2422,11 +2459,11 @@ __device__ __forceinline__ void adjoint_one(const DevNet& n, const DevWork& w, c
     const int a0 = T.inc_ptr[p], m = T.inc_split[p], z = T.inc_ptr[p + 1];
     double acc = 0.0;
     for (int e = m; e < z; ++e) {
-      const int k = inc_link(T, e);
+      const int k = T.inc[e];
       acc += s.P[k] * gQ[k];
     }
     for (int e = a0; e < m; ++e) {
-      const int k = inc_link(T, e);
+      const int k = T.inc[e];
       acc += -(s.P[k] * gQ[k]);
     }
     const int nd = n.jnode[p];
@@ -2754,13 +2791,14 @@ __device__ __forceinline__ void unrolled_one(const DevNet& n, const DevWork& w, 
     for (int p = tid; p < n.Nj; p += NT) {
       const int es = s.eslot[p];
       if (es >= 0) s.em_e[es] = rr[n.L + p];
-      s.V1[p] = rr[n.L + n.Nj + p];
     }
     gsync<NT>();
-    link_pass<NT>(n, th, T, s, rrow);
+    link_pass<NT>(n, th, T, s, rrow, w.hge + (size_t)b * n.Nj);
     gsync<NT>();
-    assemble_gga<NT, FT>(n, T, s, dj);
+    assemble_gga<NT, FT>(n, T, s, dj, w.hge + (size_t)b * n.Nj);
     factor<NT, FT>(n, T, s);  // the forward factored this matrix: positive definite
+    for (int p = tid; p < n.Nj; p += NT) s.V1[p] = rr[n.L + n.Nj + p];
+    gsync<NT>();
     // (1) q' = q - dq: the head-difference adjoint of each link
     for (int k = tid; k < n.L; k += NT) {
       const double dh = head_of(T.e1[k], s.V1, s.hf) - head_of(T.e2[k], s.V1, s.hf);
@@ -2773,8 +2811,8 @@ __device__ __forceinline__ void unrolled_one(const DevNet& n, const DevWork& w, 
     for (int p = tid; p < n.Nj; p += NT) {
       double acc = 0.0;
       const int a = T.inc_ptr[p], m = T.inc_split[p], z = T.inc_ptr[p + 1];
-      for (int e = a; e < m; ++e) acc += tl[inc_link(T, e)];
-      for (int e = m; e < z; ++e) acc += -tl[inc_link(T, e)];
+      for (int e = a; e < m; ++e) acc += tl[T.inc[e]];
+      for (int e = m; e < z; ++e) acc += -tl[T.inc[e]];
       if (last) acc += gH[n.jnode[p]];
       const int es = s.eslot[p];
       if (es >= 0) {

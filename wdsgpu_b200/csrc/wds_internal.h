@@ -124,6 +124,10 @@ struct DevNet {
   int L0, cT, nT;
   // the top block's inverse is part of the state placed by place_state
   int msm;
+  // the link pass and the top block's inversion share V1's room (place_state)
+  int join;
+  // the emitters' head losses and elevations are part of the state
+  int ems;
   // large networks: bytes of shared memory that hold the first pieces of the
   // scenario's state
   int sm_state;

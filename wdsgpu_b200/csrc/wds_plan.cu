@@ -671,28 +671,12 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
   s_md.insert(s_md.end(), md_fac.begin(), md_fac.end());
   s_md.insert(s_md.end(), md_fwd.begin(), md_fwd.end());
   s_md.insert(s_md.end(), md_bwd.begin(), md_bwd.end());
-  // incidence entries: link | PRV-with-setting << 16 | other end fixed << 17 | fixed index << 18
   std::vector<uint16_t> s_ip(inc_ptr.begin(), inc_ptr.end()), s_is(inc_split.begin(), inc_split.end());
-  std::vector<uint32_t> s_in(inc.size());
-  for (int p = 0; p < Nj; ++p)
-    for (int e = inc_ptr[p]; e < inc_ptr[p + 1]; ++e) {
-      const int k = inc[e];
-      const int other = e < inc_split[p] ? e2[k] : e1[k];
-      uint32_t v = (uint32_t)k;
-      if (net->link_kind[k] == WDS_KIND_PRV || net->link_kind[k] == WDS_KIND_FCV ||
-          net->link_kind[k] == WDS_KIND_PSV)
-        v |= 1u << 16;
-      if (other < 0) v |= (1u << 17) | ((uint32_t)(-other - 1) << 18);
-      s_in[e] = v;
-    }
+  std::vector<uint16_t> s_in(inc.begin(), inc.end());
   if (s_in.empty()) s_in.push_back(0);
   std::vector<int16_t> s_e1(e1.begin(), e1.end()), s_e2(e2.begin(), e2.end());
   std::vector<uint16_t> s_pp(pair_ptr.begin(), pair_ptr.end());
-  std::vector<uint16_t> s_pl(pair_link.size());
-  for (size_t e = 0; e < pair_link.size(); ++e)
-    s_pl[e] = (uint16_t)(pair_link[e] | ((net->link_kind[pair_link[e]] == WDS_KIND_PRV ||
-                                          net->link_kind[pair_link[e]] == WDS_KIND_FCV ||
-                                          net->link_kind[pair_link[e]] == WDS_KIND_PSV) ? 0x8000 : 0));
+  std::vector<uint16_t> s_pl(pair_link.begin(), pair_link.end());
   if (s_pl.empty()) s_pl.push_back(0);
   // ---- large networks: the levels as rounds (see factor_rounds).  Factor
   // entries: the diagonals below the top block and the entries with updates.
@@ -865,6 +849,7 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
   dsz.nxf = nxf; dsz.nT = nT;
   dsz.emcap = std::min(Nj, net->emitter_capacity > 0 ? net->emitter_capacity : 64);
   dsz.fp32 = net->factor_fp32 ? 1 : 0;
+  dsz.join = 1;
   const size_t state_bytes = state_smem_bytes(dsz);
   Blob sblob;
   TabOff to{};
@@ -983,18 +968,27 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
     plan->groups = 1;
     plan->smem_fwd = plan->smem_adj = 0;
     d.msm = d.nT > 0 ? 1 : 0;
+    d.ems = 1;
     d.sm_state = (int)std::min<size_t>(state_smem_bytes(d), 227 * 1024);
+    plan->dn_few = d;
   } else {
     // As many groups as fit (a CTA takes the SM's registers whatever its
     // count, so one CTA per SM runs).  The top block's inverse goes to shared
     // memory where that costs no group (a substitution reads it once: 4 k cycles
     // from L2, 1.5 k from shared memory, one group per SM, 36 columns), else to L2.
-    auto fits = [&](int msm, int g) {
-      d.msm = msm;
-      return (size_t)d.stab_bytes + g * state_smem_bytes(d) <= 227 * 1024;
+    // Then the emitters' losses and elevations (782 junctions with emitters at 50,
+    // 16 384 scenarios: 41.1 ms from L2, 40.4 from shared memory).  The vectors
+    // that can share room (join) do where that makes the difference.
+    auto fits = [&](DevNet& x, int msm, int ems, int g) {
+      x.msm = msm;
+      x.ems = ems;
+      for (x.join = 0; x.join < 2; ++x.join)
+        if ((size_t)x.stab_bytes + g * state_smem_bytes(x) <= 227 * 1024) return true;
+      x.join = 1;
+      return false;
     };
     int best_g = 4;
-    while (best_g > 0 && !fits(0, best_g)) --best_g;
+    while (best_g > 0 && !fits(d, 0, 0, best_g)) --best_g;
     // The order of the fewest entries can make room for one group more: taken
     // for a caller's choice that does not fit otherwise, not by itself (1300
     // junctions at 1.05 links each, one group depth-aware against two: 148
@@ -1016,7 +1010,7 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
       return WDS_PLAN_NO_FIT;
     }
     if (net->groups_per_cta > 0) {  // a tuned choice, if the state fits
-      if (!fits(0, net->groups_per_cta)) {
+      if (!fits(d, 0, 0, net->groups_per_cta)) {
         cudaFree(plan->dtab);
         delete plan;
         return fail(WDS_E_ARG, "wds_plan: groups_per_cta " + std::to_string(net->groups_per_cta) +
@@ -1025,26 +1019,23 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
       best_g = net->groups_per_cta;
       plan->tuned = true;
     }
-    const int msm = d.nT > 0 && best_g > 0 && fits(1, best_g) ? 1 : 0;
-    d.msm = msm;
+    const int top = d.nT > 0 ? 1 : 0;
+    if (!fits(d, top, 1, best_g) && !fits(d, top, 0, best_g) && !fits(d, 0, 1, best_g))
+      fits(d, 0, 0, best_g);
+    // A launch with fewer groups than the plan's (a batch below its resident
+    // scenarios) has room for all of it.
+    plan->dn_few = d;
+    if (best_g > 1 && (d.msm < top || !d.ems)) {
+      plan->few = best_g - 1;
+      while (plan->few > 0 && !fits(plan->dn_few, top, 1, plan->few)) --plan->few;
+    }
     const size_t st = state_smem_bytes(d);
     plan->groups = best_g;
     plan->smem_fwd = best_g ? (size_t)d.stab_bytes + best_g * st : (size_t)d.stab_bytes + st;
     plan->smem_adj = plan->smem_fwd;
   }
   state_offsets(d);
-  // A launch with fewer groups than the plan's (a batch below its resident
-  // scenarios) has room for the top block's inverse in shared memory.
-  plan->dn_few = d;
-  if (!d.wide && d.nT > 0 && !d.msm) {
-    DevNet& f = plan->dn_few;
-    f.msm = 1;
-    const size_t st = state_smem_bytes(f);
-    while (plan->few < plan->groups - 1 &&
-           (size_t)f.stab_bytes + (plan->few + 1) * st <= 227 * 1024)
-      ++plan->few;
-    state_offsets(f);
-  }
+  state_offsets(plan->dn_few);
   if (plan->groups == 0 || (!d.wide && plan->smem_fwd > 227 * 1024)) {
     cudaFree(plan->dtab);
     delete plan;
