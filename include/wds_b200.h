@@ -374,6 +374,12 @@ int wds_forward_noalloc(const WdsPlan* plan, int32_t batch, const WdsForwardOpts
                         double* head, double* flow, double* emitter, int8_t* status,
                         int32_t* iters, double* relerr, int32_t* info, void* stream);
 
+/* The device code's own elementary functions on n elements (device arrays; y is
+ * not read by WDS_MATH_RECIP), to measure their error: 1 / x, x / y, x ^ y. */
+enum { WDS_MATH_RECIP = 0, WDS_MATH_QUOTIENT = 1, WDS_MATH_POWER = 2 };
+int wds_math(int32_t function, int64_t n, const double* x, const double* y, double* out,
+             void* stream);
+
 /* Release the plan and its device memory. */
 int wds_free(WdsPlan* plan);
 

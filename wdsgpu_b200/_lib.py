@@ -26,8 +26,9 @@ E_NAMES = {-1: "bad argument", -2: "CUDA error", -3: "out of memory",
 EXPORTS = ("wds_plan", "wds_forward", "wds_adjoint", "wds_plan_stats",
            "wds_plan_symbolic", "wds_state_generation", "wds_free", "wds_last_error", "wds_forward_noalloc",
            "wds_forward_multi", "wds_adjoint_multi", "wds_adjoint_rhs", "wds_sensitivity", "wds_adjoint_pumps",
-           "wds_unrolled_adjoint")
+           "wds_unrolled_adjoint", "wds_math")
 MULTI_MAX = 8
+MATH_RECIP, MATH_QUOTIENT, MATH_POWER = range(3)
 
 
 class WdsNetwork(ctypes.Structure):
@@ -118,6 +119,8 @@ def load():
     lib.wds_adjoint_rhs.restype = ctypes.c_int
     lib.wds_sensitivity.argtypes = [vp, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, vp, vp, vp]
     lib.wds_sensitivity.restype = ctypes.c_int
+    lib.wds_math.argtypes = [ctypes.c_int32, ctypes.c_int64, vp, vp, vp, vp]
+    lib.wds_math.restype = ctypes.c_int
     lib.wds_adjoint_pumps.argtypes = [vp, ctypes.c_int32] + [vp] * 10 + [vp]
     lib.wds_adjoint_pumps.restype = ctypes.c_int
     lib.wds_unrolled_adjoint.argtypes = [vp, ctypes.c_int32, ctypes.c_int32] + [vp] * 4 + \

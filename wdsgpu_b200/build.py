@@ -26,6 +26,7 @@ for _k in ("forward", "adjoint", "unrolled", "multi"):
     UNITS += [("wds_k_%s.cu" % _k, "wds_k_%s_f64" % _k, ("-DWDS_FP32=0",)),
               ("wds_k_%s.cu" % _k, "wds_k_%s_f32" % _k, ("-DWDS_FP32=1",))]
 HEADERS = [os.path.join(CSRC, "wds_internal.h"), os.path.join(CSRC, "wds_device.cuh"),
+           os.path.join(CSRC, "wds_math.cuh"),
            os.path.join(REPO, "include", "wds_b200.h")]
 
 

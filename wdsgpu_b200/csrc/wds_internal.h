@@ -254,6 +254,8 @@ int launch_forward(const DevNet& n, const DevWork& w, const FwdArgs& a, int grou
                    void* stream, std::string* err);
 int launch_adjoint(const DevNet& n, const DevWork& w, const AdjArgs& a, int groups,
                    void* stream, std::string* err);
+int launch_math(int function, long long n, const double* x, const double* y, double* out,
+                void* stream, std::string* err);
 size_t state_smem_bytes(const DevNet& n);
 void state_offsets(DevNet& n);  // n.so, from the sizes, msm and sm_state
 // CTAs of a launch of the adjoint over `rows` rows (-1: a CUDA error in *err)

@@ -10,6 +10,25 @@
 
 namespace wds {
 
+namespace {
+__global__ void k_math(int function, long long n, const double* x, const double* y, double* out) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  if (function == WDS_MATH_RECIP) out[i] = recip(x[i]);
+  else if (function == WDS_MATH_QUOTIENT) out[i] = quotient(x[i], y[i], recip(y[i]));
+  else out[i] = pow_pos(x[i], y[i]);
+}
+}  // namespace
+
+int launch_math(int function, long long n, const double* x, const double* y, double* out,
+                void* stream, std::string* err) {
+  k_math<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(function, n, x, y, out);
+  const cudaError_t ce = cudaGetLastError();
+  if (ce == cudaSuccess) return WDS_OK;
+  *err = std::string("wds_math launch: ") + cudaGetErrorString(ce);
+  return WDS_E_CUDA;
+}
+
 size_t state_smem_bytes(const DevNet& n) { return smem_bytes(n); }
 void state_offsets(DevNet& n) { state_pieces(n); }
 

@@ -1376,6 +1376,16 @@ extern "C" int wds_unrolled_adjoint(WdsPlan* plan, int32_t batch, int32_t K,
   return WDS_OK;
 }
 
+extern "C" int wds_math(int32_t function, int64_t n, const double* x, const double* y,
+                        double* out, void* stream) {
+  if (function < WDS_MATH_RECIP || function > WDS_MATH_POWER || n <= 0 || n > (1LL << 31) || !x ||
+      !out || (!y && function != WDS_MATH_RECIP))
+    return fail(WDS_E_ARG, "wds_math: bad argument");
+  std::string err;
+  const int rc = wds::launch_math(function, n, x, y, out, stream, &err);
+  return rc == WDS_OK ? rc : fail(rc, err);
+}
+
 extern "C" int wds_free(WdsPlan* plan) {
   if (!plan) return WDS_OK;
   if (plan->dtab) cudaFree(plan->dtab);
