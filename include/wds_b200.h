@@ -270,7 +270,9 @@ int wds_unrolled_adjoint(WdsPlan* plan, int32_t batch, int32_t K, const double* 
                          const int8_t* status0, void* stream);
 
 /* Statistics of the plan: [Nj, nnz_L, n_levels, n_pairs, smem_bytes,
- * n_pcv, nnz_A_lower, threads]. */
+ * n_pcv, nnz_A_lower, groups per CTA].  smem_bytes: shared memory of a CTA with
+ * that many scenario groups; 0 marks the large-network layout (whose launches
+ * take up to 227 KB of shared memory for the scenario's state). */
 int wds_plan_stats(const WdsPlan* plan, int64_t* out8);
 
 /* Generation of the plan's kept state: a counter that changes with every

@@ -937,7 +937,7 @@ __device__ __noinline__ void top_apply(const double* Mg, double* vT, int nT) {
 }
 
 // Level-scheduled LDL^T.  Wide levels (many independent entries) use all the
-// group's threads and a group barrier; narrow levels run on warp 0 alone,
+// group's threads and a group barrier; narrow levels run on one warp alone,
 // separated by __syncwarp.  W holds A on entry (pattern of L, fill zero) and
 // on exit the unscaled columns L_ij D_j with 1/D_j in the diagonal slot, for
 // the columns below the top block; the top block's slots hold its Schur
@@ -1730,8 +1730,9 @@ __host__ __device__ __forceinline__ Sh place_state(const DevNet& n, Take&& take)
 // The state at `base` (shared memory on the small-network layout).  The pieces
 // lie at offsets the plan computed, kernel parameters: a piece's address is one
 // addition wherever it is used, not a register held (or spilled) from the
-// start of the scenario on (three groups: 372 -> 224 bytes of spill loads; L1
-// beside 220 KB of shared memory does not hold the spills of 768 threads).
+// start of the scenario on (three groups: 372 -> 224 bytes of spill loads with
+// the link pass of that time, 280 now; L1 beside 220 KB of shared memory does
+// not hold the spills of 768 threads).
 __device__ __forceinline__ Sh carve(const DevNet& n, unsigned char* base) {
   int i = 0;
   return place_state<false>(n, [&](size_t) { return base + n.so[i++]; });

@@ -41,7 +41,7 @@ struct ValveRec {
 // elimination index p (0..Nj-1); link ends are "end codes": p >= 0 for a
 // junction, -(f+1) for the f-th fixed-head node.
 struct DevNet {
-  int N, L, Nj, Nf, nnzL, nlev, npcv, ntl, npairs, nfill, nxf, nftask, nfpair;
+  int N, L, Nj, Nf, nnzL, nlev, npcv, npairs, nfill, nxf, nfpair;
   // links [L]
   const int8_t* kind;
   const uint8_t* flags;
@@ -78,8 +78,6 @@ struct DevNet {
   const int* pcv_link;
   const int* pcv_j1;
   const int* pcv_j2;
-  const int* pcv_off;     // slot of (j1,j2)
-  const int* pcv_xf;      // Xflow slot of jc
   const double* pcv_hset;
   const double* pcv_km;
   // the head an ACTIVE valve holds: PRV at j2 (flow enters it, sgn +1), PSV
@@ -94,15 +92,11 @@ struct DevNet {
   const int* fcv_link;
   const int* fcv_j1;
   const int* fcv_j2;
-  const int* fcv_off;     // factor slot of the (j1, j2) entry
-  const int* fcv_xf1;     // Xflow slots of its ends read by later PRVs, or -1
-  const int* fcv_xf2;
   const double* fcv_qs;   // flow setting (cfs)
   const double* fcv_km;
   // valve pass order [npcv + nfcv]: link order; v >= 0 PRV v, v < 0 FCV -1 - v
   const int* vord;
-  // tank links [ntl]
-  const int* tl_link;
+  // tank links
   const int* tl_tank;     // fixed index
   const int* tl_other;    // end code
   const double* tl_qsign;
@@ -257,12 +251,12 @@ int launch_adjoint(const DevNet& n, const DevWork& w, const AdjArgs& a, int grou
 int launch_math(int function, long long n, const double* x, const double* y, double* out,
                 void* stream, std::string* err);
 size_t state_smem_bytes(const DevNet& n);
-void state_offsets(DevNet& n);  // n.so, from the sizes, msm and sm_state
+void state_offsets(DevNet& n);  // n.so, from the sizes, msm, ems, join and sm_state
 // CTAs of a launch of the adjoint over `rows` rows (-1: a CUDA error in *err)
 int adjoint_grid(const DevNet& n, int groups, int rows, std::string* err);
 
 // One plan's share of a multi-plan launch.  `groups` is the number of
-// scenario groups (256 threads each) per 768-thread CTA; state_bytes and cta0
+// scenario groups (256 threads each) per 1024-thread CTA; state_bytes and cta0
 // are filled by the launcher.
 struct FwdJob {
   DevNet n;

@@ -171,7 +171,7 @@ struct WdsPlan {
 
 // Scenario groups per CTA of a launch of `batch` scenarios: as few as give
 // every scenario a place in the first round, up to the plan's count.  A CTA of
-// one group compiles to 255 registers per thread without spills, three groups
+// one group compiles to 190 registers per thread without spills, three groups
 // to 80 with spills, so a batch within the SM count runs faster in CTAs of one
 // group (542 junctions B=97: 289 -> 262 us of k_forward).
 static int groups_for(const WdsPlan* plan, int batch) {
@@ -381,7 +381,7 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
   // Execution mode per level and operation, one byte: bits 0-2 = log2 of the
   // lane-group size G (each item's dot product is spread over G lanes and
   // reduced with warp shuffles), bit 7 = wide (all 256 threads of the group,
-  // followed by a group barrier) instead of narrow (warp 0 only, __syncwarp).
+  // followed by a group barrier) instead of narrow (one warp, __syncwarp).
   // Cost model in units of one dependent round: rounds * (ceil(maxlen / G) +
   // 0.6 log2 G + 1), plus 0.5 per group barrier.
   const double bar_cost = net->level_barrier_cost > 0.0 ? net->level_barrier_cost : 0.5;
@@ -534,7 +534,7 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
   }
   // ---- tank links
   const int ntl = net->n_tank_links;
-  std::vector<int> link_tl(L, -1), tl_link(ntl), tl_tank(ntl), tl_other(ntl);
+  std::vector<int> link_tl(L, -1), tl_tank(ntl), tl_other(ntl);
   std::vector<double> tl_qsign(ntl), tl_hmax(ntl), tl_hmin(ntl);
   std::vector<uint8_t> tl_flags(ntl);
   for (int t = 0; t < ntl; ++t) {
@@ -542,7 +542,6 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
     if (k < 0 || k >= L || fix_idx[net->tl_tank[t]] < 0)
       return fail(WDS_E_ARG, "wds_plan: bad tank link");
     link_tl[k] = t;
-    tl_link[t] = k;
     tl_tank[t] = fix_idx[net->tl_tank[t]];
     tl_other[t] = code(net->tl_other[t]);
     tl_qsign[t] = net->tl_qsign[t];
@@ -890,14 +889,12 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
          o_el = blob.add(el), o_nxf = blob.add(xf_node), o_cbp = blob.add(cb_ptr),
          o_cbi = blob.add(cb_idx), o_fn = blob.add(fnodes), o_fincp = blob.add(finc_ptr),
          o_fincs = blob.add(finc_split), o_finc = blob.add(finc), o_pcl = blob.add(pcv_link),
-         o_pj1 = blob.add(pcv_j1), o_pj2 = blob.add(pcv_j2), o_poff = blob.add(pcv_off),
-         o_pxf = blob.add(pcv_xf), o_phs = blob.add(pcv_hset), o_pkm = blob.add(pcv_km),
-         o_tll = blob.add(tl_link), o_tlt = blob.add(tl_tank), o_tlo = blob.add(tl_other),
+         o_pj1 = blob.add(pcv_j1), o_pj2 = blob.add(pcv_j2), o_phs = blob.add(pcv_hset),
+         o_pkm = blob.add(pcv_km), o_tlt = blob.add(tl_tank), o_tlo = blob.add(tl_other),
          o_tlq = blob.add(tl_qsign), o_tlx = blob.add(tl_hmax), o_tln = blob.add(tl_hmin),
          o_tlf = blob.add(tl_flags), o_stab = blob.add(stab_bytes), o_lpu = blob.add(link_pump),
          o_phu = blob.add(phu), o_lfc = blob.add(link_fcv), o_fcl = blob.add(fcv_link),
-         o_fj1 = blob.add(fcv_j1), o_fj2 = blob.add(fcv_j2), o_fof = blob.add(fcv_off),
-         o_fx1 = blob.add(fcv_xf1), o_fx2 = blob.add(fcv_xf2), o_fqs = blob.add(fcv_qs),
+         o_fj1 = blob.add(fcv_j1), o_fj2 = blob.add(fcv_j2), o_fqs = blob.add(fcv_qs),
          o_fkm = blob.add(fcv_km), o_vord = blob.add(vord), o_pjc = blob.add(pcv_jc),
          o_pjo = blob.add(pcv_jo), o_psg = blob.add(pcv_sgn), o_pps = blob.add(pcv_psv);
   WdsPlan* plan = new WdsPlan();
@@ -915,8 +912,8 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
 #define P_(T, off) reinterpret_cast<const T*>(base + (off))
   DevNet& d = plan->dn;
   d.N = N; d.L = L; d.Nj = Nj; d.Nf = Nf; d.nnzL = nnzL; d.nlev = nlev; d.npcv = npcv;
-  d.ntl = ntl; d.npairs = (int)pair_slot.size(); d.nfill = (int)fill_slot.size(); d.nxf = nxf;
-  d.nftask = (int)ftask.size(); d.nfpair = (int)fpair.size() / 3;
+  d.npairs = (int)pair_slot.size(); d.nfill = (int)fill_slot.size(); d.nxf = nxf;
+  d.nfpair = (int)fpair.size() / 3;
   d.kind = P_(int8_t, o_kind);
   d.flags = P_(uint8_t, o_flags); d.status0 = P_(int8_t, o_st0); d.ptype = P_(int8_t, o_ptype);
   d.km = P_(double, o_km); d.km_tcv = P_(double, o_kmt); d.q_init = P_(double, o_q0);
@@ -924,8 +921,7 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
   d.pspeed = P_(double, o_psp); d.phmax = P_(double, o_phm); d.cptr = P_(int, o_cptr);
   d.phunit = P_(double, o_phu); d.link_pump = P_(int, o_lpu); d.npump = npump;
   d.nfcv = nfcv; d.link_fcv = P_(int, o_lfc); d.fcv_link = P_(int, o_fcl);
-  d.fcv_j1 = P_(int, o_fj1); d.fcv_j2 = P_(int, o_fj2); d.fcv_off = P_(int, o_fof);
-  d.fcv_xf1 = P_(int, o_fx1); d.fcv_xf2 = P_(int, o_fx2); d.fcv_qs = P_(double, o_fqs);
+  d.fcv_j1 = P_(int, o_fj1); d.fcv_j2 = P_(int, o_fj2); d.fcv_qs = P_(double, o_fqs);
   d.fcv_km = P_(double, o_fkm); d.vord = P_(int, o_vord);
   d.pcv_jc = P_(int, o_pjc); d.pcv_jo = P_(int, o_pjo); d.pcv_sgn = P_(double, o_psg);
   d.pcv_psv = P_(int, o_pps);
@@ -935,8 +931,8 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
   d.fnode = P_(int, o_fn); d.finc_ptr = P_(int, o_fincp); d.finc_split = P_(int, o_fincs);
   d.finc = P_(int, o_finc);
   d.pcv_link = P_(int, o_pcl); d.pcv_j1 = P_(int, o_pj1); d.pcv_j2 = P_(int, o_pj2);
-  d.pcv_off = P_(int, o_poff); d.pcv_xf = P_(int, o_pxf); d.pcv_hset = P_(double, o_phs);
-  d.pcv_km = P_(double, o_pkm); d.tl_link = P_(int, o_tll); d.tl_tank = P_(int, o_tlt);
+  d.pcv_hset = P_(double, o_phs);
+  d.pcv_km = P_(double, o_pkm); d.tl_tank = P_(int, o_tlt);
   d.tl_other = P_(int, o_tlo); d.tl_qsign = P_(double, o_tlq); d.tl_hmax = P_(double, o_tlx);
   d.tl_hmin = P_(double, o_tln); d.tl_flags = P_(uint8_t, o_tlf);
   d.stab = P_(uint4, o_stab);
@@ -990,10 +986,11 @@ static int plan_ordered(const WdsNetwork* net, int32_t max_batch, WdsPlan** out,
     int best_g = 4;
     while (best_g > 0 && !fits(d, 0, 0, best_g)) --best_g;
     // The order of the fewest entries can make room for one group more: taken
-    // for a caller's choice that does not fit otherwise, not by itself (1300
-    // junctions at 1.05 links each, one group depth-aware against two: 148
-    // scenarios 0.69 / 0.97 ms, 1024 3.07 / 3.35; 1100 at 1.2: 0.80 / 0.89,
-    // 3.48 / 3.00).
+    // for a caller's choice that does not fit otherwise, not by itself: it loses
+    // at batches of one round, and at several rounds it gains at one of two
+    // networks measured (1300 junctions at 1.05 links each, one group depth-aware
+    // against two: 148 scenarios 0.69 / 0.97 ms, 1024 3.07 / 3.35; 1100 at 1.2:
+    // 0.80 / 0.89, 3.48 / 3.00).
     const int want = net->groups_per_cta;
     if (!plain && !net->perm && want > best_g &&
         (size_t)d.stab_bytes + want * state_smem_bytes(d) <= 227 * 1024 * 11 / 10) {
