@@ -45,6 +45,7 @@ namespace wds {
 namespace {
 
 constexpr double kINF = __builtin_huge_val();
+constexpr double kNaN = __builtin_nan("");
 // A polish step keeps the factor in use while every link conductance P and
 // emitter term of the step is within kReuseStep (relative) of the values it
 // was factored with; the terminal state kept for the adjoint, within
@@ -285,47 +286,30 @@ __device__ __forceinline__ void valve_open(const DevNet& n, double q, double km,
   }
 }
 
-// pipe_coef by CUDA's power and plain divisions.  An infinite gradient gives
-// P = 0 and Y = NaN: the scenario does not converge, and no pivot fails.
-__device__ __noinline__ double2 pipe_any(double hexp, double rqtol, double qa, double sgn,
-                                         double r, double km) {
-  double hg = hexp * r * pow(fmax(qa, 1e-30), hexp - 1.0);
-  const bool lin = hg < rqtol;
-  if (lin) hg = rqtol;
-  double hl = lin ? hg * qa : hg * qa / hexp;
-  if (km > 0.0) {
-    hl = hl + km * qa * qa;
-    hg = hg + 2.0 * km * qa;
-  }
-  return make_double2(1.0 / hg, hl * sgn / hg);
-}
-
-// pipecoeff, Hazen-Williams / Chezy-Manning (dgga/solver.py:2176-2201)
+// pipecoeff, Hazen-Williams / Chezy-Manning (dgga/solver.py:2176-2201).  An
+// infinite gradient gives P = 0, and with it or a head loss beyond the range of
+// a double Y = NaN, as the plain divisions do (1 / inf, inf / inf): the scenario
+// does not converge, and no pivot fails.
 __device__ __forceinline__ void pipe_coef(const DevNet& n, double q, double r, double km,
                                           double& P, double& Y) {
   const double sgn = q < 0.0 ? -1.0 : 1.0;
   const double qa = q * sgn;
-  bool ok;
-  double h0 = n.hexp * r * pow_main(fmax(qa, 1e-30), n.hexp - 1.0, ok);
-  const bool lin = h0 < n.rqtol;
-  if (lin) h0 = n.rqtol;
-  const double ex = lin ? 1.0 : n.hexp, rex = lin ? 1.0 : n.rhexp;  // hl = h0 qa / ex
-  const double hg = km > 0.0 ? h0 + 2.0 * km * qa : h0;
-  // hg at 2^350 or above, infinite or NaN too: below it hg qa is finite for every
-  // r above 2^-200 (qa is below (hg / r)^(1 / (hexp - 1))), and the reciprocal's
-  // argument normal.  One rare call for the power and this: two cost 1.2 % of
-  // the kernel (782 junctions, 16 384 scenarios).
-  if (!ok || (unsigned)__double2hiint(hg) >= 0x55d00000u) {
-    const double2 c = pipe_any(n.hexp, n.rqtol, qa, sgn, r, km);
-    P = c.x;
-    Y = c.y;
-    return;
-  }
-  P = recip(hg);
-  if (km > 0.0)
-    Y = quotient(quotient(h0 * qa, ex, rex) + km * qa * qa, hg, P) * sgn;
-  else
+  double hg = n.hexp * r * pow_pos(fmax(qa, 1e-30), n.hexp - 1.0);
+  const bool lin = hg < n.rqtol;
+  if (lin) hg = n.rqtol;
+  const double ex = lin ? 1.0 : n.hexp, rex = lin ? 1.0 : n.rhexp;  // hl = hg qa / ex
+  if (km > 0.0) {
+    const double hl = quotient(hg * qa, ex, rex) + km * qa * qa;
+    hg = hg + 2.0 * km * qa;
+    P = recip(hg);
+    Y = quotient(hl, hg, P) * sgn;
+  } else {
+    P = recip(hg);
     Y = quotient(q, ex, rex);
+  }
+  // by selects: a rare call instead costs the four-group kernel 7 %
+  P = hg == kINF ? 0.0 : P;
+  Y = hg * qa < kINF ? Y : kNaN;
 }
 
 // Pump parameters of one scenario: rows of [L] values read at pump links
@@ -1731,7 +1715,7 @@ __host__ __device__ __forceinline__ Sh place_state(const DevNet& n, Take&& take)
 // lie at offsets the plan computed, kernel parameters: a piece's address is one
 // addition wherever it is used, not a register held (or spilled) from the
 // start of the scenario on (three groups: 372 -> 224 bytes of spill loads with
-// the link pass of that time, 280 now; L1 beside 220 KB of shared memory does
+// the link pass of that time, 248 now; L1 beside 220 KB of shared memory does
 // not hold the spills of 768 threads).
 __device__ __forceinline__ Sh carve(const DevNet& n, unsigned char* base) {
   int i = 0;

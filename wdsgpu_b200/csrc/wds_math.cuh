@@ -35,11 +35,11 @@ __device__ __noinline__ double pow_any(double x, double y) { return pow(x, y); }
 // then y (e + log2 m) = n + g and 2^g = e^(g ln 2) likewise.  The coefficients
 // are Chebyshev interpolants of (atanh(s) / s - 1) / s^2 on [0, 0.0295] in s^2
 // (as rounded, 2^-60.6 of log2 m) and of (e^t - 1 - t) / t^2 on +-ln(2) / 2
-// (2^-61.3 of the result).  `ok` is false, and the value void, for arguments that
-// are not positive, normal and finite and for results near the ends of the range.
-__device__ __forceinline__ double pow_main(double x, double y, bool& ok) {
+// (2^-61.3 of the result).  Arguments that are not positive, normal and finite,
+// and results near the ends of the range, take CUDA's function.
+__device__ __forceinline__ double pow_pos(double x, double y) {
   const int hx = __double2hiint(x);
-  ok = (unsigned)(hx - 0x00100000) < 0x7fe00000u;
+  if ((unsigned)(hx - 0x00100000) >= 0x7fe00000u) return pow_any(x, y);
   const int e = (hx - 0x3fe6a09f) >> 20;
   const double m = __hiloint2double(hx - (e << 20), __double2loint(x));
   const double f = m - 1.0, d = f + 2.0, dl = f - (d - 2.0);  // m + 1 = d + dl
@@ -62,7 +62,7 @@ __device__ __forceinline__ double pow_main(double x, double y, bool& ok) {
   const double b0 = E + hi, b1 = ((E - b0) + hi) + lo;
   const double b = b0 + b1, bl = (b0 - b) + b1;  // log2 x
   const double ph = y * b, pl = fma(y, bl, fma(y, b, -ph));
-  ok = ok && fabs(ph) < 1000.0;
+  if (!(fabs(ph) < 1000.0)) return pow_any(x, y);
   const double nm = ph + 0x1.8p52;
   const int n = __double2loint(nm);  // ph to the nearest integer
   const double g = ph - (nm - 0x1.8p52);
@@ -82,12 +82,6 @@ __device__ __forceinline__ double pow_main(double x, double y, bool& ok) {
   const double a = 1.0 + t, w = t * t * q;
   const double v = a + fma(tl, a + w, ((1.0 - a) + t) + w);
   return __hiloint2double(__double2hiint(v) + (n << 20), __double2loint(v));
-}
-// ... which take CUDA's function.
-__device__ __forceinline__ double pow_pos(double x, double y) {
-  bool ok;
-  const double v = pow_main(x, y, ok);
-  return ok ? v : pow_any(x, y);
 }
 
 }  // namespace

@@ -81,8 +81,7 @@ def sensitivity_matrix(solver, demand, res_head, r_hw, sensor_nodes, wrt="C", fr
     fr = list(range(B)) if frames is None else [int(b) for b in frames]
     rows = B * m
     # a negative index counts from the last node, as it does in numpy
-    sens_t = torch.as_tensor(np.where(sensors < 0, sensors + s.N, sensors).astype(np.int32),
-                             device=dev)
+    sens_t = torch.as_tensor((sensors % s.N).astype(np.int32), device=dev)
     chain = torch.as_tensor(dr_dC_chain(s, r_hw), device=dev) if wrt == "C" else None
     cur = torch.cuda.current_stream(dev)
     t1 = perf_counter()
