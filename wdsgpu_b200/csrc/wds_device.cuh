@@ -292,8 +292,7 @@ __device__ __forceinline__ void valve_open(const DevNet& n, double q, double km,
 // does not converge, and no pivot fails.
 __device__ __forceinline__ void pipe_coef(const DevNet& n, double q, double r, double km,
                                           double& P, double& Y) {
-  const double sgn = q < 0.0 ? -1.0 : 1.0;
-  const double qa = q * sgn;
+  const double qa = fabs(q);
   double hg = n.hexp * r * pow_pos(fmax(qa, 1e-30), n.hexp - 1.0);
   const bool lin = hg < n.rqtol;
   if (lin) hg = n.rqtol;
@@ -302,7 +301,7 @@ __device__ __forceinline__ void pipe_coef(const DevNet& n, double q, double r, d
     const double hl = quotient(hg * qa, ex, rex) + km * qa * qa;
     hg = hg + 2.0 * km * qa;
     P = recip(hg);
-    Y = quotient(hl, hg, P) * sgn;
+    Y = copysign(quotient(hl, hg, P), q);
   } else {
     P = recip(hg);
     Y = quotient(q, ex, rex);
