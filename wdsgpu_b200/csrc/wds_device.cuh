@@ -822,8 +822,8 @@ __device__ __forceinline__ void top_steps(int nT, int tiles, int w, int lane,
 // where four single-column sweeps on 3 x 3 entries per thread cost 48
 // multiplies and FMAs per lane and four barriers of the whole group.  A
 // seventh warp inverts the pivot blocks (44 columns, alone / three groups per
-// SM: 19.0 / 31.3 k cycles with the single-column sweeps, 11.2 / 16.8 k so).
-// What bounds it is the chain of a
+// SM: 19.0 / 31.3 k cycles with the single-column sweeps, 11.2 / 16.8 k so with
+// pivots in pairs, under 1 % more now).  What bounds it is the chain of a
 // block: publish the columns, invert the 4 x 4 block (four reciprocals), read
 // it back, update the next block's tile.  S is read from the factor slots
 // listed in dslot, S^{-1} is written to Mg (row-major, rows of top_ld(nT)
