@@ -8,6 +8,7 @@ import torch
 from oracle.gga import Model
 from wdsgpu_b200 import GGASolver, implicit_solve, synth
 from wdsgpu_b200.autodiff import solve_unrolled
+from wdsgpu_b200.multi import implicit_solve_multi
 
 pytestmark = pytest.mark.gpu
 
@@ -89,3 +90,20 @@ def test_results_do_not_depend_on_where_the_state_lies(cuda, nj, links, emitters
             out += [x.detach() for x in o[:3]] + [D.grad, K.grad]
         res.append(out)
     assert all(torch.equal(x, y) for x, y in zip(*res))
+
+
+def test_networks_that_just_fit_in_one_launch(cuda):
+    # the multi-network launch takes the plans' own placement: as each alone
+    ss, D, RH, alone = [], [], [], []
+    for case in ((540, 648, 270), (425, 850, 0)):
+        net, d, rh = _case(*case, B=3)
+        s = GGASolver(net, device=cuda, dense_status_machine=True)
+        ss.append(s)
+        D.append(torch.tensor(d, device=cuda, requires_grad=True))
+        RH.append(torch.tensor(rh, device=cuda))
+        h = implicit_solve(s, D[-1], RH[-1], accuracy=1e-7)[0]
+        alone.append((h.detach(), torch.autograd.grad((h ** 2).sum(), D[-1])[0]))
+    out = implicit_solve_multi(ss, D, RH, accuracy=1e-7)
+    grads = torch.autograd.grad(sum((o[0] ** 2).sum() for o in out), D)
+    for (h, g), o, gm in zip(alone, out, grads):
+        assert torch.equal(h, o[0]) and torch.equal(g, gm)
